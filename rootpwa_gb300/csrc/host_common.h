@@ -140,12 +140,12 @@ using namespace pwa;
 // ampIntegralMatrix: raw sums and the wave list
 // ===========================================================================
 // device buffers and stream of integrate(), kept by an integral between
-// calls on one device (the output matrix, the error flag and the Gram
-// partials: no allocation per call once they have their size)
+// calls on one device (the output matrix, the error flag, the Gram partials
+// and the rows' range: no allocation per call once they have their size)
 struct GramScratch {
 	int dev = -1;
 	cudaStream_t stream = nullptr;
-	DevBuf out, err, part;
+	DevBuf out, err, part, rowMax;
 	GramScratch() = default;
 	GramScratch(const GramScratch&) = delete;
 	GramScratch& operator=(const GramScratch&) = delete;
@@ -155,6 +155,7 @@ struct GramScratch {
 		out.release();
 		err.release();
 		part.release();
+		rowMax.release();
 		if (stream)
 			cudaStreamDestroy(stream);
 		stream = nullptr;

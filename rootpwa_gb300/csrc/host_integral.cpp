@@ -13,7 +13,8 @@ namespace {
 
 // Sums the GPU Gram kernel for integrate().
 int gramOnDevice(GramScratch& sc, uint32_t W, const void* amps, uint64_t nEvents, uint32_t nSub, int ampType,
-                 int memory, const std::vector<double>& weightK, uint64_t K, int precision, std::vector<cplx>& out)
+                 int memory, const std::vector<double>& weightK, bool weights01, uint64_t K, int precision,
+                 std::vector<cplx>& out)
 {
 	int dev, sms;
 	size_t smem;
@@ -109,14 +110,14 @@ int gramOnDevice(GramScratch& sc, uint32_t W, const void* amps, uint64_t nEvents
 		if (st != kOk)
 			return st;
 	} else {
-		const int tps = ((int)W + 63) / 64;
-		const int nTiles = tps * (tps + 1) / 2;
-		int chunks = std::max(1, (4 * sms + nTiles - 1) / nTiles);
-		const uint64_t maxChunks = std::max<uint64_t>(1, K / 64);
-		chunks = (int)std::min<uint64_t>((uint64_t)chunks, maxChunks);
+		const int chunks = gramSimtChunks(g, precision, sms);
 		g.chunks = chunks;
 		PWA_TRY(dPart.ensure((size_t)chunks * W * W * 2 * sizeof(double), "gram partials"));
-		PWA_TRY(cudaCheck(cudaMemsetAsync(dPart.p, 0, (size_t)chunks * W * W * 2 * sizeof(double), s), "memset"));
+		if (precision == PWA_PRECISION_FP64) {
+			PWA_TRY(sc.rowMax.ensure((1 + (size_t)chunks * W) * sizeof(unsigned), "row range"));
+			g.rowMax = sc.rowMax.as<unsigned>();
+		}
+		g.weights01 = weights01;
 		g.partials = dPart.as<double>();
 		PWA_TRY(launchGramSimt(g, precision, s));
 		PWA_TRY(launchGramReduce(g.partials, chunks, (int)W, dOut.as<double>(), 0, s));
@@ -255,8 +256,8 @@ int pwa_integral_integrate(pwa_integral* I, uint32_t nWaves, const char* const* 
 			I->scratch.p.reset(new (std::nothrow) GramScratch());
 		if (!I->scratch.p)
 			return setError(kErrOom, "out of host memory");
-		PWA_TRY(gramOnDevice(*I->scratch.p, nWaves, amps, nEvents, nSubAmps, ampType, memory, weightK, K, precision,
-		                     result));
+		PWA_TRY(gramOnDevice(*I->scratch.p, nWaves, amps, nEvents, nSubAmps, ampType, memory, weightK, !useWeight, K,
+		                     precision, result));
 	} else {
 		result.assign((size_t)nWaves * nWaves, cplx(0, 0));
 	}
