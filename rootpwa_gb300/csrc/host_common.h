@@ -140,12 +140,12 @@ using namespace pwa;
 // ampIntegralMatrix: raw sums and the wave list
 // ===========================================================================
 // device buffers and stream of integrate(), kept by an integral between
-// calls on one device (the output matrix, the error flag, the Gram partials
-// and the rows' range: no allocation per call once they have their size)
+// calls on one device (the output matrix, the error flag, the Gram partials,
+// the rows' range and the event weights: no allocation per call once they have their size)
 struct GramScratch {
 	int dev = -1;
 	cudaStream_t stream = nullptr;
-	DevBuf out, err, part, rowMax;
+	DevBuf out, err, part, rowMax, weights, rawWeights;
 	GramScratch() = default;
 	GramScratch(const GramScratch&) = delete;
 	GramScratch& operator=(const GramScratch&) = delete;
@@ -156,6 +156,8 @@ struct GramScratch {
 		err.release();
 		part.release();
 		rowMax.release();
+		weights.release();
+		rawWeights.release();
 		if (stream)
 			cudaStreamDestroy(stream);
 		stream = nullptr;

@@ -184,12 +184,11 @@ __device__ __forceinline__ float2 fmul2(float2 a, float2 b)
 // a warp, whose J are consecutive, read consecutive 16-byte pieces.
 __device__ __forceinline__ float4 ldOp(const float2* p) { return *reinterpret_cast<const float4*>(p); }
 
-__device__ __forceinline__ void triConvert(float2& d, float2 v) { d = v; }
-template <typename In>
-__device__ __forceinline__ void triConvert(double2& d, In v) { d = make_double2((double)v.x, (double)v.y); }
-__device__ __forceinline__ void triScale(float2& d, float2 v, float w) { d = make_float2(v.x * w, v.y * w); }
-template <typename In>
-__device__ __forceinline__ void triScale(double2& d, In v, double w) { d = make_double2((double)v.x * w, (double)v.y * w); }
+// 8 bytes from global to shared memory in the background, or zeros
+__device__ __forceinline__ void copyAsync8(void* dst, const void* src, bool valid)
+{
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smemAddr(dst)), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
 
 // one staged row of a slice: element offset of its first amplitude, steps of
 // K it has, position of its first operand (24 bits) and slice
@@ -204,7 +203,8 @@ struct __align__(16) TriSlot {
 struct AccF32 {
 	typedef float2 Op;
 	typedef float Weight;
-	static constexpr int kCols = 4, kPrefetch = 6, kFold = 1 << 30;
+	static constexpr int kCols = 4, kUnroll = 2, kFold = 1 << 30;
+	static constexpr bool kAsync = true;
 	float2 s[4][4];
 	__device__ void init(const unsigned*, int, int, int)
 	{
@@ -213,7 +213,8 @@ struct AccF32 {
 				s[p][q] = make_float2(0.f, 0.f);
 	}
 	static __device__ __forceinline__ int pos(int G, int row) { return ((((row >> 1) & 1) * G + (row >> 2)) << 1) | (row & 1); }
-	__device__ void step(const float2* A, const float2* B, int G, int I, int J)
+	template <bool WT>
+	__device__ void step(const float2* A, const float2* B, int G, int I, int J, float w)
 	{
 		float2 a[4], b[4];
 #pragma unroll
@@ -226,6 +227,8 @@ struct AccF32 {
 		}
 #pragma unroll
 		for (int p = 0; p < 4; ++p) {
+			if (WT)
+				a[p] = make_float2(a[p].x * w, a[p].y * w);
 			const float2 ar = make_float2(a[p].y, -a[p].x);
 #pragma unroll
 			for (int q = 0; q < 4; ++q) {
@@ -241,7 +244,8 @@ struct AccF32 {
 struct AccF64 {
 	typedef double2 Op;
 	typedef double Weight;
-	static constexpr int kCols = 4, kPrefetch = 2, kFold = 1 << 30;  // the FP64 pipe hides the loads
+	static constexpr int kCols = 4, kUnroll = 2, kFold = 1 << 30;
+	static constexpr bool kAsync = false;
 	double2 s[4][4];
 	__device__ void init(const unsigned*, int, int, int)
 	{
@@ -250,7 +254,8 @@ struct AccF64 {
 				s[p][q] = make_double2(0., 0.);
 	}
 	static __device__ __forceinline__ int pos(int G, int row) { return (row & 3) * G + (row >> 2); }
-	__device__ void step(const double2* A, const double2* B, int G, int I, int J)
+	template <bool WT>
+	__device__ void step(const double2* A, const double2* B, int G, int I, int J, double)
 	{
 		double2 a[4], b[4];
 #pragma unroll
@@ -275,7 +280,8 @@ struct AccF64 {
 struct AccLevels {
 	typedef float2 Op;
 	typedef float Weight;
-	static constexpr int kCols = 2, kPrefetch = 4, kFold = kLevelFold;
+	static constexpr int kCols = 2, kUnroll = 4, kFold = kLevelFold;
+	static constexpr bool kAsync = true;
 	float2 s[4][2], u[4][2], c[4][2];  // on the two grids, below them
 	double2 d[4][2];
 	int eRow[4], eCol[2];  // components of the row are below 2^e
@@ -314,13 +320,16 @@ struct AccLevels {
 		u = v;
 		c = fsub2(fadd2(c, r), ne);
 	}
-	__device__ void step(const float2* A, const float2* B, int, int I, int J)
+	template <bool WT>
+	__device__ void step(const float2* A, const float2* B, int, int I, int J, float w)
 	{
 		const float4 x = ldOp(A + 4 * I), y = ldOp(A + 4 * I + 2), z = ldOp(B + 2 * J);
-		const float2 a[4] = {make_float2(x.x, x.y), make_float2(x.z, x.w), make_float2(y.x, y.y), make_float2(y.z, y.w)};
+		float2 a[4] = {make_float2(x.x, x.y), make_float2(x.z, x.w), make_float2(y.x, y.y), make_float2(y.z, y.w)};
 		const float2 b[2] = {make_float2(z.x, z.y), make_float2(z.z, z.w)};
 #pragma unroll
 		for (int p = 0; p < 4; ++p) {
+			if (WT)  // 0 or 1
+				a[p] = make_float2(a[p].x * w, a[p].y * w);
 			const float2 na = make_float2(-a[p].x, -a[p].y);
 			const float2 ar = make_float2(a[p].y, na.x), nar = make_float2(na.y, a[p].x);
 #pragma unroll
@@ -404,13 +413,15 @@ struct TriArgs {
 };
 
 // One block: `slices` chunks of K, one thread tile per thread.  KT steps of
-// K are staged per round in two buffers; the next round's amplitudes are
-// loaded into registers while this one is used.
+// K are staged per round in two buffers: the FP32 operands by asynchronous
+// copies that run while the previous round is used (held in registers for
+// that time, they spilled: 250 against 130 us at 50 waves), the FP64 ones
+// converted and weighted on the way, beside which the FP64 pipe hides their
+// loads.
 template <typename Acc, typename In, int KT, bool WT>
 __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __restrict__ amps, const TriArgs a)
 {
 	typedef typename Acc::Op Op;
-	constexpr int NP = Acc::kPrefetch;  // prefetched amplitudes per thread
 	extern __shared__ __align__(16) unsigned char smemRaw[];
 	if (a.outside && *a.outside != a.runOutside)
 		return;
@@ -429,8 +440,12 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 	J += kUnits * I;
 	const bool mine = sl < a.slices && t < a.nTiles;
 	const int G = a.g - I0, rows = 4 * G;        // staged groups and rows
-	const int stepOps = KT * rows;               // operands of a slice
-	const int bufOps = a.slices * stepOps * (WT ? 2 : 1);
+	// a step's operands are an odd number of 16-byte pieces, so that the KT
+	// threads which stage a row store to different banks
+	constexpr int kPad = 16 / sizeof(Op);
+	const int ld = rows + kPad, stepOps = KT * ld;
+	constexpr bool kTwo = WT && !Acc::kAsync;  // weighted copies beside the operands
+	const int bufOps = a.slices * stepOps * (kTwo ? 2 : 1);
 	Op* const buf0 = reinterpret_cast<Op*>(smemRaw);
 	const uint64_t chunk0 = (uint64_t)blockIdx.y * (unsigned)a.slices;
 	Acc acc;
@@ -456,78 +471,75 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 	const uint64_t wk0 = (chunk0 + tid / KT) * a.chunkLen + (tid & (KT - 1));
 	auto weight = [&](uint32_t kb) {
 		const uint64_t k = wk0 + kb;
-		return (wMine && kb + (tid & (KT - 1)) < a.chunkLen && k < a.K) ? (typename Acc::Weight)a.weightK[k]
-		                                                                : (typename Acc::Weight)0;
+		return (wMine && kb + (tid & (KT - 1)) < a.chunkLen && k < a.K) ? a.weightK[k] : 0.;
 	};
 	if (wMine) {
-		wbuf[tid] = weight(0);
-		wbuf[a.slices * KT + tid] = weight(KT);
+		wbuf[tid] = (typename Acc::Weight)weight(0);
+		wbuf[a.slices * KT + tid] = (typename Acc::Weight)weight(KT);
 	}
 	__syncthreads();
-	// thread: step kk of rows tid / KT, + rowStep, ...; the first NP of them
-	// are loaded a round ahead
+	// thread: step kk of rows tid / KT, + rowStep, ...
 	const int kk = tid & (KT - 1), rowStep = nThreads / KT;
-	auto fetch = [&](int n, uint32_t kb) {
-		const TriSlot z = slots[n];
-		In v{0, 0};
-		if (kb + kk < z.lim)
-			v = amps[z.off + kb + kk];
-		return v;
-	};
-	auto place = [&](Op* buf, int n, In v, int round) {
-		const uint32_t base = slots[n].base;
-		Op* d = buf + (base & 0xffffffu) + kk * rows;
-		triConvert(*d, v);
-		if (WT)
-			triScale(d[a.slices * stepOps], v, wbuf[((round & 1) * a.slices + (base >> 24)) * KT + kk]);
-	};
-	In pv[NP];
-	auto prefetch = [&](uint32_t kb) {
-#pragma unroll
-		for (int x = 0; x < NP; ++x) {
-			const int n = tid / KT + x * rowStep;
-			if (n < total)
-				pv[x] = fetch(n, kb);
+	auto stage = [&](Op* buf, uint32_t kb, int round) {
+		for (int n = tid / KT; n < total; n += rowStep) {
+			const TriSlot z = slots[n];
+			Op* d = buf + (z.base & 0xffffffu) + kk * ld;
+			const bool valid = kb + kk < z.lim;
+			const In* src = amps + (valid ? z.off + kb + kk : 0);
+			if constexpr (Acc::kAsync) {
+				copyAsync8(d, src, valid);
+			} else {
+				In v{0, 0};
+				if (valid)
+					v = *src;
+				*d = Op{(double)v.x, (double)v.y};
+				if (kTwo) {
+					const double w = wbuf[((round & 1) * a.slices + (z.base >> 24)) * KT + kk];
+					d[a.slices * stepOps] = Op{(double)v.x * w, (double)v.y * w};
+				}
+			}
 		}
+		if constexpr (Acc::kAsync)
+			asm volatile("cp.async.commit_group;" ::: "memory");
 	};
-	auto commit = [&](Op* buf, uint32_t kb, int round) {
-#pragma unroll
-		for (int x = 0; x < NP; ++x) {
-			const int n = tid / KT + x * rowStep;
-			if (n < total)
-				place(buf, n, pv[x], round);
-		}
-		for (int n = tid / KT + NP * rowStep; n < total; n += rowStep)
-			place(buf, n, fetch(n, kb), round);
+	auto arrived = [&]() {
+		if constexpr (Acc::kAsync)
+			asm volatile("cp.async.wait_group 0;" ::: "memory");
+		__syncthreads();
 	};
 
-	prefetch(0);
-	commit(buf0, 0, 0);
-	__syncthreads();
+	stage(buf0, 0, 0);
+	arrived();
 	const uint32_t len = (uint32_t)a.chunkLen;
 	int cur = 0, sinceFold = 0;
 	for (uint32_t kb = 0, round = 0; kb < len; kb += KT, ++round) {
 		const bool more = kb + KT < len;
-		if (more)
-			prefetch(kb + KT);
-		const typename Acc::Weight wNext = weight(kb + 2 * KT);
+		Op* const next = buf0 + (cur ^ 1) * bufOps;
+		if (Acc::kAsync && more)
+			stage(next, kb + KT, round + 1);
+		const double wNext = weight(kb + 2 * KT);
 		if (mine) {
 			const Op* b0 = buf0 + cur * bufOps + sl * stepOps;
-			const Op* a0 = WT ? b0 + a.slices * stepOps : b0;
-#pragma unroll 2
+			const Op* a0 = kTwo ? b0 + a.slices * stepOps : b0;
+			const typename Acc::Weight* w0 = wbuf + ((round & 1) * a.slices + sl) * KT;
+#pragma unroll Acc::kUnroll
 			for (int q = 0; q < KT; ++q)
-				acc.step(a0 + q * rows, b0 + q * rows, G, I - I0, J - kUnits * I0);
+				acc.template step<WT>(a0 + q * ld, b0 + q * ld, G, I - I0, J - kUnits * I0, WT ? w0[q] : 0);
 			sinceFold += KT;
 			if (Acc::kFold < (1 << 30) && (sinceFold == Acc::kFold || !more)) {
 				sinceFold = 0;
 				acc.fold();
 			}
 		}
-		if (more)
-			commit(buf0 + (cur ^ 1) * bufOps, kb + KT, round + 1);
-		if (wMine)
-			wbuf[(round & 1) * a.slices * KT + tid] = wNext;  // of round + 2
-		__syncthreads();
+		if (!Acc::kAsync && more)
+			stage(next, kb + KT, round + 1);
+		// round + 2's weights replace this round's, which have been read: by
+		// the staging in the last round, or else when all threads arrive
+		if (!Acc::kAsync && wMine)
+			wbuf[(round & 1) * a.slices * KT + tid] = (typename Acc::Weight)wNext;
+		arrived();
+		if (Acc::kAsync && wMine)
+			wbuf[(round & 1) * a.slices * KT + tid] = (typename Acc::Weight)wNext;
 		cur ^= 1;
 	}
 	if (!mine || chunk0 + sl >= (uint64_t)a.chunks)
@@ -593,7 +605,7 @@ constexpr size_t kTriSmemMax = 112 * 1024;  // two blocks per SM
 // shared memory of one chunk: two rounds of operands, the row table, weights
 size_t triSliceBytes(int g, int KT, size_t opBytes, bool weighted)
 {
-	return (size_t)2 * KT * 4 * g * opBytes * (weighted ? 2 : 1) + (size_t)4 * g * sizeof(TriSlot) +
+	return (size_t)2 * KT * (4 * g * opBytes + 16) * (weighted && opBytes == sizeof(double2) ? 2 : 1) + (size_t)4 * g * sizeof(TriSlot) +
 	       2 * KT * sizeof(double);
 }
 
@@ -717,6 +729,41 @@ int launchGramSimt(const GramArgs& a, int precision, cudaStream_t s)
 	}
 	countLaunches(1);
 	return cudaCheck(cudaGetLastError(), "gram SIMT launch");
+}
+
+// weights of importance-sampled events (ampIntegralMatrix.cc:408-429): a
+// block takes a contiguous run of events, its threads strided compensated
+// sums combined in a fixed order
+__global__ void __launch_bounds__(256) inverseWeightsKernel(const double* __restrict__ w, uint64_t n, uint32_t nSub,
+                                                            double* out, double* sums)
+{
+	__shared__ double part[256];
+	const uint64_t run = (n + gridDim.x - 1) / gridDim.x, k0 = blockIdx.x * run, k1 = min(n, k0 + run);
+	double sum = 0., comp = 0.;
+	for (uint64_t k = k0 + threadIdx.x; k < k1; k += 256) {
+		const double v = 1. / w[k];
+		for (uint32_t s = 0; s < nSub; ++s)
+			out[k * nSub + s] = v;
+		const double y = v - comp, t = sum + y;
+		comp = (t - sum) - y;
+		sum = t;
+	}
+	part[threadIdx.x] = sum - comp;
+	__syncthreads();
+	for (int o = 128; o > 0; o >>= 1) {
+		if ((int)threadIdx.x < o)
+			part[threadIdx.x] += part[threadIdx.x + o];
+		__syncthreads();
+	}
+	if (threadIdx.x == 0)
+		sums[blockIdx.x] = part[0];
+}
+
+int launchInverseWeights(const double* w, uint64_t n, uint32_t nSub, double* out, double* sums, cudaStream_t s)
+{
+	inverseWeightsKernel<<<kWeightBlocks, 256, 0, s>>>(w, n, nSub, out, sums);
+	countLaunches(1);
+	return cudaCheck(cudaGetLastError(), "weights launch");
 }
 
 // out += the blocks of a Gram of two row groups: rows and columns i < G of

@@ -171,6 +171,10 @@ int gramSimtChunks(const GramArgs& a, int precision, int numSMs);
 int launchGramSimt(const GramArgs& a, int precision, cudaStream_t s);
 // out = (accumulate ? out : 0) + sum of chunk partials, mirrored to the lower triangle
 int launchGramReduce(const double* partials, int chunks, int W, double* out, int accumulate, cudaStream_t s);
+// out[ev * nSub + s] = 1 / w[ev] and, per block, the compensated sum of 1 / w
+// of its events into sums[kWeightBlocks]
+constexpr int kWeightBlocks = 152;
+int launchInverseWeights(const double* w, uint64_t n, uint32_t nSub, double* out, double* sums, cudaStream_t s);
 // out[w] = sum_k a[w][k] for W complex64 rows of n elements (row stride ld),
 // FP64 (complex128 out[W])
 int launchRowSums(const float2* a, uint64_t n, uint64_t ld, int W, double* out, cudaStream_t s);
