@@ -45,47 +45,48 @@ int uploadPlan(pwa_isobar* A)
 	                   A->reflection, A->canonical, A->isospinSym ? &A->isospin : nullptr, p);
 	if (!why.empty())
 		return setError(kErrArg, why);
-	const size_t oWaves = 0;
-	const size_t oOrder = align16(oWaves + p.waves.size() * sizeof(iso::WaveDev));
-	const size_t oLams = align16(oOrder + p.order.size() * sizeof(int32_t));
-	const size_t oTerms = align16(oLams + p.lams.size() * sizeof(iso::LamTerm));
-	const size_t oPoly = align16(oTerms + p.dterms.size() * sizeof(iso::DTerm));
-	const size_t oNorm = align16(oPoly + sizeof(p.bfPoly));
-	const size_t oPolyF = align16(oNorm + sizeof(p.bfNorm));
-	const size_t oNormF = align16(oPolyF + sizeof(p.bfPolyF));
-	const size_t oPerms = align16(oNormF + sizeof(p.bfNormF));
-	const size_t oTermsS = align16(oPerms + p.perms.size() * sizeof(int32_t));
-	const size_t total = align16(oTermsS + p.terms.size() * sizeof(iso::SymTerm));
-	std::vector<unsigned char> h(total, 0);
-	auto put = [&](size_t off, const void* src, size_t bytes) {
-		if (bytes)
-			std::memcpy(h.data() + off, src, bytes);
-	};
-	put(oWaves, p.waves.data(), p.waves.size() * sizeof(iso::WaveDev));
-	put(oOrder, p.order.data(), p.order.size() * sizeof(int32_t));
-	put(oLams, p.lams.data(), p.lams.size() * sizeof(iso::LamTerm));
-	put(oTerms, p.dterms.data(), p.dterms.size() * sizeof(iso::DTerm));
-	put(oPoly, p.bfPoly, sizeof(p.bfPoly));
-	put(oNorm, p.bfNorm, sizeof(p.bfNorm));
-	put(oPolyF, p.bfPolyF, sizeof(p.bfPolyF));
-	put(oNormF, p.bfNormF, sizeof(p.bfNormF));
-	put(oPerms, p.perms.data(), p.perms.size() * sizeof(int32_t));
-	put(oTermsS, p.terms.data(), p.terms.size() * sizeof(iso::SymTerm));
-	PWA_TRY(A->dPlan.ensure(total, "isobar wave plan"));
-	PWA_TRY(cudaCheck(cudaMemcpyAsync(A->dPlan.p, h.data(), total, cudaMemcpyHostToDevice, A->stream), "plan upload"));
-	PWA_TRY(cudaCheck(cudaStreamSynchronize(A->stream), "plan upload"));
-	unsigned char* d = A->dPlan.as<unsigned char>();
+	// the arrays one after the other, 16-byte aligned; `fix` moves the view's
+	// pointers to them once the buffer exists
+	std::vector<unsigned char> h;
+	std::vector<std::pair<size_t, const void**>> fix;
 	iso::PlanView v = p.view();
-	v.waves = reinterpret_cast<const iso::WaveDev*>(d + oWaves);
-	v.order = reinterpret_cast<const int32_t*>(d + oOrder);
-	v.lams = reinterpret_cast<const iso::LamTerm*>(d + oLams);
-	v.dterms = reinterpret_cast<const iso::DTerm*>(d + oTerms);
-	v.bfPoly = reinterpret_cast<const double*>(d + oPoly);
-	v.bfNorm = reinterpret_cast<const double*>(d + oNorm);
-	v.bfPolyF = reinterpret_cast<const float*>(d + oPolyF);
-	v.bfNormF = reinterpret_cast<const float*>(d + oNormF);
-	v.perms = reinterpret_cast<const int32_t*>(d + oPerms);
-	v.terms = reinterpret_cast<const iso::SymTerm*>(d + oTermsS);
+	auto put = [&](const void* src, size_t bytes, const void** at) {
+		h.resize(align16(h.size()));
+		fix.push_back(std::make_pair(h.size(), at));
+		h.insert(h.end(), static_cast<const unsigned char*>(src), static_cast<const unsigned char*>(src) + bytes);
+	};
+#define PUT(member) put(p.member.data(), p.member.size() * sizeof(p.member[0]), (const void**)&v.member)
+	PUT(waves);
+	PUT(batches);
+	PUT(insts);
+	PUT(eops);
+	PUT(isoWave);
+	PUT(phaseM);
+	PUT(lxL);
+	PUT(fams);
+	PUT(dops);
+	PUT(coef);
+	PUT(coefF);
+	PUT(angs);
+	PUT(xops);
+	PUT(xopsF);
+	PUT(lams);
+	PUT(lamsF);
+	PUT(waveOps);
+	PUT(factors);
+	PUT(factorsF);
+	PUT(perms);
+#undef PUT
+	put(p.bfPoly, sizeof(p.bfPoly), (const void**)&v.bfPoly);
+	put(p.bfNorm, sizeof(p.bfNorm), (const void**)&v.bfNorm);
+	put(p.bfPolyF, sizeof(p.bfPolyF), (const void**)&v.bfPolyF);
+	put(p.bfNormF, sizeof(p.bfNormF), (const void**)&v.bfNormF);
+	h.resize(align16(h.size()) + 16);
+	PWA_TRY(A->dPlan.ensure(h.size(), "isobar wave plan"));
+	PWA_TRY(cudaCheck(cudaMemcpyAsync(A->dPlan.p, h.data(), h.size(), cudaMemcpyHostToDevice, A->stream), "plan upload"));
+	PWA_TRY(cudaCheck(cudaStreamSynchronize(A->stream), "plan upload"));
+	for (const auto& f : fix)
+		*f.second = A->dPlan.as<unsigned char>() + f.first;
 	A->devView = v;
 	A->dirty = false;
 	return kOk;

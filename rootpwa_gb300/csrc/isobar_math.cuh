@@ -84,70 +84,111 @@ constexpr double kVesF0Mass = 0.9837, kVesF0Width = 0.0376, kVesCouplingRe = -0.
 struct DTerm {
 	double coef;
 	int32_t a, b;
-	float coefF;                    // coef in FP32 (complex64 mode)
-	int32_t pad;
 };
 
-// one spin projection of the isobar in one wave: the X-vertex angular part
-// cPlus e^{i mPlus phi/2} dPlus(theta) + cMinus e^{i mMinus phi/2} dMinus(theta)
-// (couplings, norms and the reflectivity combination folded into cPlus,
-// cMinus) times the isobar vertex e^{i lamIso phiH/2} dIso(thetaH).
-// Helicity formalism: mPlus/mMinus = +-M, dPlus/dMinus = d^J_{+-M lam},
-// dIso = d^j_{lam 0}.  Canonical formalism: mPlus/mMinus = +-M - m,
-// dPlus/dMinus = d^L_{+-M-m, 0} (spherical harmonics Y_L), dIso = d^l_{m 0}.
-struct LamTerm {
-	int32_t lamIso;                 // 2 lambda (helicity) or 2 m (canonical) of the isobar
-	int32_t plus0, plus1;           // DTerm range of dPlus
-	int32_t minus0, minus1;         // DTerm range of dMinus (empty if unused)
-	int32_t iso0, iso1;             // DTerm range of dIso
-	int32_t mPlus, mMinus;          // phase multipliers (units of 1/2)
-	double cPlus, cMinus;
-	float cPlusF, cMinusF;          // FP32 copies (complex64 mode)
-};
-
+// what the mass dependence and the barrier factor of a wave's isobar need
 struct WaveDev {
 	int32_t a, b, c;                // isobar daughters 1, 2 and the bachelor (final-state slots)
 	int32_t bachelorFirst;          // X-vertex daughter 1 (the analyser) is the bachelor
-	int32_t M;                      // 2M of X
 	int32_t LX, LI;                 // 2L of the X and isobar vertices (barrier factors)
 	int32_t massDep;
+	int32_t q0Zero;                 // q0 == 0 (the relativistic Breit-Wigner is then 0)
 	double m0, g0;                  // isobar mass and width (binned: the bin's lower and upper edge)
 	double q0, f2q0;                // breakup momentum at m0 and F_L^2(q0) (relativistic BW)
 	double ma, mb;                  // isobar daughter masses
 	double q02;                     // breakup momentum squared at m0 (rho BW)
+	double kG;                      // g0 m0^2 / (q0 f2q0) (relativistic BW)
 	double mdp[10];                 // parameters of the K pi S-wave forms
-	int32_t lam0, lam1;             // LamTerm range
-	int32_t term0, term1;           // SymTerm range (symmetrisation terms)
-	int32_t topo;                   // topology class (waves of one class share kinematics)
-	int32_t iso;                    // isobar class: waves of equal mass dependence and isobar L
-	int32_t q0Zero;                 // q0 == 0 (the relativistic Breit-Wigner is then 0)
 	// FP32 copies for the complex64 mode, whose per-wave arithmetic must not
 	// convert FP64 constants (a conversion runs on the FP64 pipe)
-	float m0F, g0F, q0F, f2q0F, maF, mbF, q02F;
+	float m0F, g0F, q0F, maF, mbF, q02F, kGF;
 	float dmHi, dmLo;               // the mass M that M^2 - m^2 is formed with (m0; Flatte: its M0), hi + lo
 };
 
-// one symmetrisation term of a wave: final-state permutation (index into the
-// six permutations of three slots) and its factor (Bose times isospin)
-struct SymTerm {
-	int32_t perm;
-	float factorF;                  // factor in FP32 (complex64 mode)
-	double factor;
+// The amplitude of a wave for one symmetrisation term is
+//   factor x iso x lx x sum over the isobar's spin projections lam of
+//     (cP e^{i M phi/2} dP(theta) + cM e^{-i M phi/2} dM(theta)) E_lam
+// with iso = mass dependence x isobar barrier factor, lx the X vertex's
+// barrier factor and E_lam the isobar vertex e^{i lam phiH/2} d_lam(thetaH)
+// (canonical formalism: times e^{-i lam phi/2}, which leaves the X vertex the
+// phases +-M as well).  Few of these factors are a wave's own: the 88 waves of
+// a 3pi wave set have 16 E_lam, 9 families of at most seven real d functions,
+// some 70 X-vertex sums up to a factor, 6 iso, 5 lx and 76 sums over lam.  The
+// plan is a program that evaluates each once per event and term into a table:
+// batches of waves of one topology class, in a batch families of waves that
+// share their d functions, in a family the sums over lam and the waves of
+// each.  "at" marks table entries; complex ones are even.
+
+// sum_k coef[k] c^(a - 2k) s^(b + 2k) = c^(a - 2n + 2) s^b x (homogeneous in c^2, s^2)
+struct alignas(16) DOp {
+	int32_t coef0, n;               // coefficients
+	int32_t c, s;                   // powers of cos and sin that factor out
+};
+struct alignas(16) EOp {
+	DOp d;
+	int32_t lam, pad[3];            // 2 lam
+};
+// x = a dP + r dM, y = a dP - r dM  ->  (x cos(M phi/2), y sin(M phi/2))
+template <typename T>
+struct alignas(16) XOp {
+	T a, r;
+	int32_t dP, dM;                 // at
+	int32_t phase, negM;            // at (-1: M = 0); sign of M
+};
+// coef X E
+template <typename T>
+struct alignas(16) LamOp {
+	T coef;
+	int32_t x, e;                   // at
+};
+struct alignas(16) AngOp {
+	int32_t lam0, lam1;             // LamOp range
+	int32_t lx, wave1;              // at; end of its WaveOps (they follow those of the sum before)
+};
+struct alignas(16) WaveOp {
+	int32_t wave, iso;              // row of the result; at
+	int32_t factor0, pad;           // factors by instance
+};
+struct alignas(16) FamOp {
+	int32_t d0, d1, x0, x1;         // DOp and XOp ranges
+	int32_t ang0, ang1, pad[2];     // AngOp range
+};
+struct Batch {
+	int32_t a, b, c, bachelorFirst;
+	int32_t inst0, nInst;           // instances: permutations in `insts`
+	int32_t pow;                    // highest power of cos, sin
+	int32_t e0, e1, iso0, iso1, phase0, phase1, lx0, lx1, fam0, fam1, wave0;
+	int32_t atC, atS, atE, atIso, atPhase, atX, atLx, atD;
 };
 
 // read-only view of a wave plan (device or host pointers)
 struct PlanView {
 	const WaveDev* waves;
-	const int32_t* order;           // waves sorted by topology class
-	const LamTerm* lams;
-	const DTerm* dterms;
+	const Batch* batches;
+	const int32_t* insts;           // permutation of every instance
+	const EOp* eops;
+	const int32_t* isoWave;         // a wave of every isobar class
+	const int32_t* phaseM;          // 2M
+	const int32_t* lxL;             // 2L
+	const FamOp* fams;
+	const DOp* dops;
+	const double* coef;
+	const float* coefF;
+	const AngOp* angs;
+	const XOp<double>* xops;
+	const XOp<float>* xopsF;
+	const LamOp<double>* lams;
+	const LamOp<float>* lamsF;
+	const WaveOp* waveOps;
+	const double* factors;          // [WaveOp][instance]
+	const float* factorsF;
 	const double* bfPoly;           // [8][8]: P_l(z) coefficients of z^0..z^l
 	const double* bfNorm;           // [8]: P_l(1)
 	const float* bfPolyF;           // FP32 copies (complex64 mode)
 	const float* bfNormF;
 	const int32_t* perms;           // [6][3]: the permutations of three slots; slot i takes particle perms[p][i]
-	const SymTerm* terms;
-	uint32_t nWaves, pad0;
+	uint32_t nWaves, nBatches;
+	int32_t maxInst, tableSize;     // instances of a batch; table entries
 	double masses[3], beamMass;
 	int32_t spaceInversion, reflection;
 	int32_t canonical;              // isobar rest frame by a boost alone (canonical formalism)
@@ -155,7 +196,7 @@ struct PlanView {
 };
 
 template <typename T>
-struct C2T {
+struct alignas(2 * sizeof(T)) C2T {
 	T re, im;
 };
 typedef C2T<double> C2;
@@ -212,8 +253,12 @@ PWA_HD double vdot(V3 u, V3 v) { return u.x * v.x + u.y * v.y + u.z * v.z; }
 PWA_HD V3 vcross(V3 u, V3 v) { return V3{u.y * v.z - u.z * v.y, u.z * v.x - u.x * v.z, u.x * v.y - u.y * v.x}; }
 PWA_HD V3 vunit(V3 u)
 {
-	const double n = sqrt(vdot(u, u));
-	return n > 0 ? vscale(u, 1.0 / n) : u;
+	const double n2 = vdot(u, u);
+#if defined(__CUDA_ARCH__)
+	return n2 > 0 ? vscale(u, rsqrt(n2)) : u;
+#else
+	return n2 > 0 ? vscale(u, 1.0 / std::sqrt(n2)) : u;
+#endif
 }
 
 struct LV {
@@ -223,10 +268,12 @@ struct LV {
 
 // (e, p) in the rest frame of (eX, pX) of mass mX:
 // e' = (e eX - p.pX) / mX,  p' = p - pX (e + e') / (eX + mX)
-PWA_HD LV toRest(LV v, V3 pX, double eX, double mX)
+// (imX = 1 / mX, iem = 1 / (eX + mX): FP64 divisions are long sequences on the
+// narrow FP64 pipe, and several vectors share these)
+PWA_HD LV toRest(LV v, V3 pX, double eX, double imX, double iem)
 {
-	const double e1 = (v.e * eX - vdot(v.p, pX)) / mX;
-	return LV{vadd(v.p, vscale(pX, -(v.e + e1) / (eX + mX))), e1};
+	const double e1 = (v.e * eX - vdot(v.p, pX)) * imX;
+	return LV{vadd(v.p, vscale(pX, -(v.e + e1) * iem)), e1};
 }
 
 template <typename T>
@@ -247,7 +294,7 @@ PWA_HD T dEval(const DTerm* t, int t0, int t1, T c, T s)
 {
 	T d = T(0);
 	for (int k = t0; k < t1; ++k)
-		d += pick<T>(t[k].coef, t[k].coefF) * ipow(c, t[k].a) * ipow(s, t[k].b);
+		d += T(t[k].coef) * ipow(c, t[k].a) * ipow(s, t[k].b);
 	return d;
 }
 
@@ -266,18 +313,37 @@ PWA_HD double bfNormAt<double>(const PlanView& P, int l) { return P.bfNorm[l]; }
 template <>
 PWA_HD float bfNormAt<float>(const PlanView& P, int l) { return P.bfNormF[l]; }
 
-// Blatt-Weisskopf F_L(q)^2 = P_l(1) z^l / P_l(z), z = (q / 0.1973)^2, L = 2l
+// Blatt-Weisskopf F_L(q)^2 = P_l(1) z^l / P_l(z), z = (q / 0.1973)^2, L = 2l:
+// numerator and denominator.  Up to l = 3 without loops (zero coefficients
+// above l), whose loads and branches cost more than the arithmetic.
+template <typename T>
+PWA_HD T barrierParts(const PlanView& P, int L, T q2, T* den)
+{
+	const int l = L / 2;
+	if (l == 0) {
+		*den = T(1);
+		return T(1);
+	}
+	const T z = q2 * T(1.0 / (kPr * kPr));
+	if (l <= 3) {
+		const T c0 = bfPolyAt<T>(P, 8 * l), c1 = bfPolyAt<T>(P, 8 * l + 1), c2 = bfPolyAt<T>(P, 8 * l + 2),
+		        c3 = bfPolyAt<T>(P, 8 * l + 3);
+		*den = c0 + z * (c1 + z * (c2 + z * c3));
+		const T zl = l == 1 ? z : l == 2 ? z * z : z * z * z;
+		return bfNormAt<T>(P, l) * zl;
+	}
+	T d = bfPolyAt<T>(P, 8 * l + l);
+	for (int k = l - 1; k >= 0; --k)
+		d = d * z + bfPolyAt<T>(P, 8 * l + k);
+	*den = d;
+	return bfNormAt<T>(P, l) * ipow(z, l);
+}
 template <typename T>
 PWA_HD T barrierF2(const PlanView& P, int L, T q)
 {
-	const int l = L / 2;
-	if (l == 0)
-		return T(1);
-	const T z = (q * q) / T(kPr * kPr);
-	T den = bfPolyAt<T>(P, 8 * l + l);
-	for (int k = l - 1; k >= 0; --k)
-		den = den * z + bfPolyAt<T>(P, 8 * l + k);
-	return bfNormAt<T>(P, l) * ipow(z, l) / den;
+	T den;
+	const T num = barrierParts<T>(P, L, q * q, &den);
+	return num / den;
 }
 
 template <typename T>
@@ -288,12 +354,13 @@ PWA_HD T breakup2(T M, T m1, T m2)
 }
 
 // 2 k / m with the complex breakup momentum k of two particles of mass m1
-// (imaginary below threshold, physUtils.hpp:108-120)
-PWA_HD C2T<double> rhoOf(double m, double m1)
+// (imaginary below threshold, physUtils.hpp:108-120); (2 k / m)^2 =
+// (m - 2 m1) (m + 2 m1) / m^2, is2 = 1 / m^2
+PWA_HD C2T<double> rhoOf(double m, double is2, double m1)
 {
-	const double q2 = breakup2<double>(m, m1, m1);
-	const double r = 2.0 * sqrt(q2 < 0 ? -q2 : q2) / m;
-	return q2 < 0 ? C2T<double>{0.0, r} : C2T<double>{r, 0.0};
+	const double r2 = (m - 2.0 * m1) * (m + 2.0 * m1) * is2;
+	const double r = sqrt(r2 < 0 ? -r2 : r2);
+	return r2 < 0 ? C2T<double>{0.0, r} : C2T<double>{r, 0.0};
 }
 
 // KPiSGLASS::amp (massDependence.cc:700-722): LASS-type K pi S-wave,
@@ -358,22 +425,23 @@ PWA_HD C2T<double> piPiSWave(double m, int variant)
 		m += 1e-6;
 		s = m * m;
 	}
+	const double is2 = 1.0 / s;
 	C2T<double> rho;
 	if (variant == kMassPiPiSVes) {
-		rho = rhoOf(m, kMassPiCharged);
+		rho = rhoOf(m, is2, kMassPiCharged);
 	} else {
-		const C2T<double> rc = rhoOf(m, kMassPiCharged), rn = rhoOf(m, kMassPiNeutral);
+		const C2T<double> rc = rhoOf(m, is2, kMassPiCharged), rn = rhoOf(m, is2, kMassPiNeutral);
 		rho = C2T<double>{0.5 * (rc.re + rn.re), 0.5 * (rc.im + rn.im)};
 	}
 	const double mk = 0.5 * (kMassKCharged + kMassKNeutral);
-	const double scale = s / (4.0 * mk * mk) - 1.0;
+	const double scale = s * (1.0 / (4.0 * mk * mk)) - 1.0;
 	const bool kachaev = variant == kMassPiPiSKachaev;
 	double M = kAmpA0 / (s - kAmpS0) + (kachaev ? 0.0 : kAmpF1 * kAmpF1 / (s - kAmpS1));
 	const double x = scale, x2 = x * x;
 	M += kAmpC0 + kAmpC1 * x + kAmpC2 * x2 + kAmpC3 * x2 * x + (kachaev ? 0.0 : kAmpC4 * x2 * x2);
 	// 1 / (M - i rho) = 1 / ((M + Im rho) - i Re rho)
-	const double dRe = M + rho.im, dIm = -rho.re, n2 = dRe * dRe + dIm * dIm;
-	C2T<double> amp{dRe / n2, -dIm / n2};
+	const double dRe = M + rho.im, dIm = -rho.re, in2 = 1.0 / (dRe * dRe + dIm * dIm);
+	C2T<double> amp{dRe * in2, -dIm * in2};
 	if (variant == kMassPiPiSVes && m > 2.0 * kMassPiCharged) {
 		const double q = sqrt(breakup2<double>(m, kMassPiCharged, kMassPiCharged));
 		const double q0 = sqrt(breakup2<double>(kVesF0Mass, kMassPiCharged, kMassPiCharged));
@@ -398,10 +466,13 @@ PWA_HD C2T<T> massDependence(const PlanView& P, const WaveDev& w, T mI, T dm2, d
 	if (w.massDep == kMassRelBw) {
 		if (w.q0Zero)
 			return C2T<T>{T(0), T(0)};
-		const T q2 = breakup2<T>(mI, ma, mb);
-		const T q = q2 > T(0) ? sqrt(q2) : T(0);
-		const T G = g0 * (m0 / mI) * (q / q0) * (barrierF2<T>(P, w.LI, q) / pick<T>(w.f2q0, w.f2q0F));
-		const T A = m0 * g0, B = dm2, Cc = m0 * G;
+		// m0 Gamma = g0 m0^2 / (q0 F^2(q0)) q F^2(q) / m
+		const T rm = T(1) / mI;
+		const T q2r = (mI - (ma + mb)) * (mI + (ma + mb)) * (mI - (ma - mb)) * (mI + (ma - mb)) * (T(0.25) * rm * rm);
+		const T q2 = q2r > T(0) ? q2r : T(0);
+		T den;
+		const T num = barrierParts<T>(P, w.LI, q2, &den);
+		const T A = m0 * g0, B = dm2, Cc = pick<T>(w.kG, w.kGF) * sqrt(q2) * rm * (num / den);
 		const T f = A / (B * B + Cc * Cc);
 		return C2T<T>{f * B, f * Cc};
 	}
@@ -481,24 +552,7 @@ struct Kin {
 	T cI, sI, c2I, s2I, qI;
 	T mI, mIlo;                     // isobar mass in T; FP32: mI + mIlo is the FP64 mass to ~2^-48
 	double mId;                     // isobar mass in FP64
-	// values shared by the waves of this kinematics, cached on first use:
-	// the mass dependence of the isobar mass alone (by mass-dependence kind),
-	// mass dependence x sqrt(F_LI(qI)) (by isobar class), sqrt(F_LX(qX)) (by LX)
-	int32_t mdKind, isoKey, lxKey;
-	C2T<T> md, isoVal;
-	T lxVal;
-	PWA_HD void clearCaches()
-	{
-		mdKind = isoKey = lxKey = -1;
-	}
 };
-
-// mass dependences that depend on the isobar mass alone (no per-wave
-// parameters): evaluated once per topology class and symmetrisation term
-PWA_HD bool massDepOfMassAlone(int k)
-{
-	return k == kMassF0980Flatte || k == kMassRhoPrime || (k >= kMassPiPiSM && k <= kMassPiPiSKachaev);
-}
 
 PWA_HD double phiOf(double x, double y) { return (x == 0.0 && y == 0.0) ? 0.0 : atan2(y, x); }
 
@@ -515,15 +569,10 @@ PWA_HD void halfAngle(double perp, double z, double* c, double* s)
 
 // angles from FP64 components, evaluated in FP32 (the complex64 mode: the
 // per-wave arithmetic that consumes them is FP32)
-PWA_HD float phiOfF(double x, double y)
-{
-	const float xf = (float)x, yf = (float)y;
-	return (xf == 0.f && yf == 0.f) ? 0.f : atan2f(yf, xf);
-}
+PWA_HD float phiOfF(float xf, float yf) { return (xf == 0.f && yf == 0.f) ? 0.f : atan2f(yf, xf); }
 
-PWA_HD void halfAngleF(double x, double y, double z, float* c, float* s, float* q)
+PWA_HD void halfAngleF(float xf, float yf, float zf, float* c, float* s, float* q)
 {
-	const float xf = (float)x, yf = (float)y, zf = (float)z;
 	const float perp = sqrtf(xf * xf + yf * yf);
 	const float th = (perp == 0.f && zf == 0.f) ? 0.f : atan2f(perp, zf);
 	float sf, cf;
@@ -538,38 +587,37 @@ PWA_HD void halfAngleF(double x, double y, double z, float* c, float* s, float* 
 	*q = sqrtf(perp * perp + zf * zf);
 }
 
-// g: the Gottfried-Jackson four-vectors of the final-state slots of one
-// symmetrisation term.  T = double: FP64 throughout.  T = float (complex64
+// A, B, Cb: the Gottfried-Jackson four-vectors of the isobar's daughters and of
+// the bachelor in one symmetrisation term.  T = double: FP64 throughout.  T = float (complex64
 // amplitudes): the boosts, the isobar mass and momentum and the helicity
 // frame's boost along z stay in FP64 (they cancel); the angles and
 // magnitudes the per-wave FP32 arithmetic consumes are computed in FP32
 // from the FP64 components, which keeps GB300's narrow FP64 pipe off the
 // transcendental functions.
 template <typename T>
-PWA_HD Kin<T> kinematics(const LV g[3], const WaveDev& w, bool canonical);
+PWA_HD Kin<T> kinematics(const LV& A, const LV& B, const LV& Cb, bool bachelorFirst, bool canonical);
 
 template <>
-PWA_HD Kin<float> kinematics<float>(const LV g[3], const WaveDev& w, bool canonical)
+PWA_HD Kin<float> kinematics<float>(const LV& A, const LV& B, const LV& Cb, bool bachelorFirst, bool canonical)
 {
-	const LV A = g[w.a], B = g[w.b], Cb = g[w.c];
 	const LV I{vadd(A.p, B.p), A.e + B.e};
 	Kin<float> k;
-	k.clearCaches();
-	const V3 d1 = w.bachelorFirst ? Cb.p : I.p;
-	k.u = cexpi(0.5f * phiOfF(d1.x, d1.y));
-	halfAngleF(d1.x, d1.y, d1.z, &k.cX, &k.sX, &k.qX);
+	const V3 d1 = bachelorFirst ? Cb.p : I.p;
+	const float dx = (float)d1.x, dy = (float)d1.y;
+	k.u = cexpi(0.5f * phiOfF(dx, dy));
+	halfAngleF(dx, dy, (float)d1.z, &k.cX, &k.sX, &k.qX);
 	k.c2X = k.cX * k.cX;
 	k.s2X = k.sX * k.sX;
 	const double pI = sqrt(vdot(I.p, I.p));
 	k.mId = sqrt((I.e - pI) * (I.e + pI));
 	k.mI = (float)k.mId;
 	k.mIlo = (float)(k.mId - (double)k.mI);
-	double ax, ay, az;
+	float ax, ay, az;
 	if (canonical) {
-		const LV r = toRest(A, I.p, I.e, k.mId);
-		ax = r.p.x;
-		ay = r.p.y;
-		az = r.p.z;
+		const LV r = toRest(A, I.p, I.e, 1.0 / k.mId, 1.0 / (I.e + k.mId));
+		ax = (float)r.p.x;
+		ay = (float)r.p.y;
+		az = (float)r.p.z;
 	} else {
 		// helicity frame: transverse axes in FP32, the boost along z in FP64
 		const float ix = (float)I.p.x, iy = (float)I.p.y, iz = (float)I.p.z;
@@ -585,7 +633,7 @@ PWA_HD Kin<float> kinematics<float>(const LV g[3], const WaveDev& w, bool canoni
 		const float axf = (float)A.p.x, ayf = (float)A.p.y, azf = (float)A.p.z;
 		ax = axf * xx + ayf * xy + azf * xz;
 		ay = axf * yx + ayf * yy;
-		az = (I.e * (vdot(A.p, I.p) / pI) - pI * A.e) / k.mId;
+		az = (float)((I.e * vdot(A.p, I.p) - vdot(I.p, I.p) * A.e) / (pI * k.mId));
 	}
 	k.uH = cexpi(0.5f * phiOfF(ax, ay));
 	halfAngleF(ax, ay, az, &k.cI, &k.sI, &k.qI);
@@ -595,13 +643,11 @@ PWA_HD Kin<float> kinematics<float>(const LV g[3], const WaveDev& w, bool canoni
 }
 
 template <>
-PWA_HD Kin<double> kinematics<double>(const LV g[3], const WaveDev& w, bool canonical)
+PWA_HD Kin<double> kinematics<double>(const LV& A, const LV& B, const LV& Cb, bool bachelorFirst, bool canonical)
 {
-	const LV A = g[w.a], B = g[w.b], Cb = g[w.c];
 	const LV I{vadd(A.p, B.p), A.e + B.e};
 	Kin<double> k;
-	k.clearCaches();
-	const V3 d1 = w.bachelorFirst ? Cb.p : I.p;
+	const V3 d1 = bachelorFirst ? Cb.p : I.p;
 	const double perp1 = sqrt(d1.x * d1.x + d1.y * d1.y);
 	k.u = cexpi(0.5 * phiOf(d1.x, d1.y));
 	halfAngle(perp1, d1.z, &k.cX, &k.sX);
@@ -615,7 +661,7 @@ PWA_HD Kin<double> kinematics<double>(const LV g[3], const WaveDev& w, bool cano
 	if (canonical) {
 		// rest frame of the isobar with the Gottfried-Jackson axes
 		// (isobarCanonicalAmplitude.cc:94-108)
-		const LV r = toRest(A, I.p, I.e, k.mI);
+		const LV r = toRest(A, I.p, I.e, 1.0 / k.mI, 1.0 / (I.e + k.mI));
 		ax = r.p.x;
 		ay = r.p.y;
 		az = r.p.z;
@@ -672,100 +718,19 @@ PWA_HD C2T<T> cpowi(C2T<T> u, int m)
 	return r;
 }
 
-// d^j_{m n}(theta) from its Wigner terms t0..t1-1 (dEval's arguments): the
-// power of cos(theta/2) falls and that of sin(theta/2) rises by 2 from one
-// term to the next (wignerTerms), so the sum is c^a_last s^b_first times a
-// homogeneous polynomial in c^2 and s^2, evaluated Horner-like
-template <typename T>
-PWA_HD T dHorner(const DTerm* t, int t0, int t1, T c, T s, T c2, T s2)
-{
-	if (t0 >= t1)
-		return T(0);
-	T r = pick<T>(t[t0].coef, t[t0].coefF), sk = T(1);
-	for (int k = t0 + 1; k < t1; ++k) {
-		sk *= s2;
-		r = r * c2 + pick<T>(t[k].coef, t[k].coefF) * sk;
-	}
-	return r * ipow(c, t[t1 - 1].a) * ipow(s, t[t0].b);
-}
-
-// amplitude of wave w for one symmetrisation term; T is the arithmetic of
-// the per-wave part.  k is the term's kinematics; the values that several
-// waves share (mass dependence and isobar barrier factor of one isobar class,
-// the X-vertex barrier factor of one L) are cached in it.
-template <typename T>
-PWA_HD C2T<T> termAmplitude(const PlanView& P, const WaveDev& w, Kin<T>& k)
-{
-	// e^{i lamIso phiH / 2} as a power of e^{i phiH / 2}, stepped by e^{i phiH}
-	const C2T<T> stepH = cmul(k.uH, k.uH);
-	C2T<T> eL{T(1), T(0)};
-	C2T<T> sum{T(0), T(0)};
-	// e^{i m phi / 2} of the X vertex, recomputed only when m changes
-	// (helicity formalism: m = +-M for every isobar helicity of the wave)
-	constexpr int kNone = 1 << 30;
-	int mP = kNone, mM = kNone;
-	C2T<T> eP{T(1), T(0)}, eM{T(1), T(0)};
-	for (int t = w.lam0; t < w.lam1; ++t) {
-		const LamTerm& L = P.lams[t];
-		if (t == w.lam0)
-			eL = cpowi(k.uH, L.lamIso);
-		else
-			for (int s = P.lams[t - 1].lamIso; s < L.lamIso; s += 2)
-				eL = cmul(eL, stepH);
-		C2T<T> x{T(0), T(0)};
-		if (L.plus1 > L.plus0) {
-			if (L.mPlus != mP) {
-				mP = L.mPlus;
-				eP = cpowi(k.u, mP);
-			}
-			x = cscale(eP, pick<T>(L.cPlus, L.cPlusF) * dHorner<T>(P.dterms, L.plus0, L.plus1, k.cX, k.sX, k.c2X, k.s2X));
-		}
-		if (L.minus1 > L.minus0) {
-			if (L.mMinus != mM) {
-				mM = L.mMinus;
-				eM = (mP != kNone && mM == -mP) ? C2T<T>{eP.re, -eP.im} : cpowi(k.u, mM);
-			}
-			x = cadd(x, cscale(eM, pick<T>(L.cMinus, L.cMinusF) *
-			                           dHorner<T>(P.dterms, L.minus0, L.minus1, k.cX, k.sX, k.c2X, k.s2X)));
-		}
-		const T dI = dHorner<T>(P.dterms, L.iso0, L.iso1, k.cI, k.sI, k.c2I, k.s2I);
-		sum = cadd(sum, cmul(x, cscale(eL, dI)));
-	}
-	if (k.isoKey != w.iso) {
-		C2T<T> md;
-		if (massDepOfMassAlone(w.massDep)) {
-			if (k.mdKind != w.massDep) {
-				k.md = massDependence<T>(P, w, k.mI, deltaM2(w, k), k.mId);
-				k.mdKind = w.massDep;
-			}
-			md = k.md;
-		} else {
-			md = massDependence<T>(P, w, k.mI, deltaM2(w, k), k.mId);
-		}
-		k.isoVal = cscale(md, static_cast<T>(sqrt(barrierF2<T>(P, w.LI, k.qI))));
-		k.isoKey = w.iso;
-	}
-	if (k.lxKey != w.LX) {
-		k.lxVal = static_cast<T>(sqrt(barrierF2<T>(P, w.LX, k.qX)));
-		k.lxKey = w.LX;
-	}
-	return cscale(cmul(sum, k.isoVal), k.lxVal);
-}
-
 // Gottfried-Jackson four-vectors of the three final-state slots of one
-// event and symmetrisation term: beam momentum bp, final-state momenta fp
-// (lab); slot i takes the momentum of particle perm[i] and keeps its own
-// mass (decayTopology::revertMomenta with particle::setMomentum), so X and
-// the frame follow the permutation when it exchanges particles of different
-// mass (isospin partners)
-PWA_HD void gjFrame(const PlanView& P, const double bp[3], const double fp[3][3], const int32_t* perm, LV g[3])
+// event and symmetrisation term: beam momentum bp, the slots' momenta fp
+// (lab); in a permuted term slot i has the momentum of particle perm[i] and
+// keeps its own mass (decayTopology::revertMomenta with
+// particle::setMomentum), so X and the frame follow the permutation when it
+// exchanges particles of different mass (isospin partners)
+PWA_HD void gjFrame(const PlanView& P, const double bp[3], const double fp[3][3], LV g[3])
 {
 	LV f[3];
 	V3 pX{0.0, 0.0, 0.0};
 	double eX = 0.0;
 	for (int i = 0; i < 3; ++i) {
-		const int k = perm[i];
-		f[i].p = V3{fp[k][0], fp[k][1], fp[k][2]};
+		f[i].p = V3{fp[i][0], fp[i][1], fp[i][2]};
 		f[i].e = sqrt(P.masses[i] * P.masses[i] + vdot(f[i].p, f[i].p));
 		pX = vadd(pX, f[i].p);
 		eX += f[i].e;
@@ -774,61 +739,202 @@ PWA_HD void gjFrame(const PlanView& P, const double bp[3], const double fp[3][3]
 	const double mX = sqrt((eX - pXa) * (eX + pXa));
 	const V3 b{bp[0], bp[1], bp[2]};
 	const LV beam{b, sqrt(P.beamMass * P.beamMass + vdot(b, b))};
-	const V3 z = vunit(toRest(beam, pX, eX, mX).p);
+	const double imX = 1.0 / mX, iem = 1.0 / (eX + mX);
+	const V3 z = vunit(toRest(beam, pX, eX, imX, iem).p);
 	const V3 y = vunit(vcross(b, pX));
 	const V3 x = vcross(y, z);
 	const double sgn = P.spaceInversion ? -1.0 : 1.0;
 	const double sgnY = P.reflection ? -sgn : sgn;
 	for (int i = 0; i < 3; ++i) {
-		const LV r = toRest(f[i], pX, eX, mX);
+		const LV r = toRest(f[i], pX, eX, imX, iem);
 		g[i] = LV{V3{sgn * vdot(r.p, x), sgnY * vdot(r.p, y), sgn * vdot(r.p, z)}, r.e};
 	}
 }
 
-// all waves of one event; out is complex [wave][ld] as interleaved T
-// (complex128 for T = double, complex64 for T = float: FP64 frames and
-// kinematics, per-wave arithmetic in T)
+// four coefficients of a d function (lists are padded to fours)
 template <typename T>
-PWA_HD void eventAmplitudes(const PlanView& P, const double bp[3], const double fp[3][3], T* out, uint64_t ld,
-                            uint64_t e)
+struct alignas(16) Coef4 {
+	T c[4];
+};
+template <typename T>
+PWA_HD Coef4<T> coefAt(const PlanView& P, int i);
+template <>
+PWA_HD Coef4<double> coefAt<double>(const PlanView& P, int i) { return reinterpret_cast<const Coef4<double>*>(P.coef)[i >> 2]; }
+template <>
+PWA_HD Coef4<float> coefAt<float>(const PlanView& P, int i) { return reinterpret_cast<const Coef4<float>*>(P.coefF)[i >> 2]; }
+template <typename T>
+PWA_HD LamOp<T> lamAt(const PlanView& P, int i);
+template <>
+PWA_HD LamOp<double> lamAt<double>(const PlanView& P, int i) { return P.lams[i]; }
+template <>
+PWA_HD LamOp<float> lamAt<float>(const PlanView& P, int i) { return P.lamsF[i]; }
+template <typename T>
+PWA_HD XOp<T> xopAt(const PlanView& P, int i);
+template <>
+PWA_HD XOp<double> xopAt<double>(const PlanView& P, int i) { return P.xops[i]; }
+template <>
+PWA_HD XOp<float> xopAt<float>(const PlanView& P, int i) { return P.xopsF[i]; }
+
+// the table of one event and instance: entries 2i, 2i + 1 side by side, pairs
+// 2 x stride apart
+template <typename T>
+struct Table {
+	T* tab;
+	int stride;
+	PWA_HD T get(int i) const { return tab[(i & ~1) * stride + (i & 1)]; }
+	PWA_HD void set(int i, T v) const { tab[(i & ~1) * stride + (i & 1)] = v; }
+	PWA_HD C2T<T> getc(int i) const { return *reinterpret_cast<const C2T<T>*>(tab + i * stride); }
+	PWA_HD void setc(int i, C2T<T> v) const { *reinterpret_cast<C2T<T>*>(tab + i * stride) = v; }
+	// 1, x, x^2, .., x^n at i ..
+	PWA_HD void powers(int i, T x, int n) const
+	{
+		T v = T(1);
+		for (int k = 0; k <= n; ++k) {
+			set(i + k, v);
+			v *= x;
+		}
+	}
+};
+
+// a d function from the powers of cos and sin in the table, Horner-like in
+// c^2 and s^2 (the power of cos(theta/2) falls and that of sin(theta/2) rises
+// by 2 from one of Wigner's terms to the next)
+template <typename T>
+PWA_HD T dValue(const PlanView& P, const Batch& B, const DOp& d, const Table<T>& t, T c2, T s2)
 {
-	// the frame of the unpermuted event; a permutation that only exchanges
-	// particles of equal mass (Bose terms) permutes its four-vectors
-	LV g0[3];
-	gjFrame(P, bp, fp, P.perms, g0);
-	// kinematics per permutation, computed once per topology class on first use
-	Kin<T> kin[kMaxPerms];
-	uint32_t valid = 0;
-	int topo = -1;
-	for (uint32_t o = 0; o < P.nWaves; ++o) {
-		const int wi = P.order[o];
-		const WaveDev& w = P.waves[wi];
-		if (w.topo != topo) {
-			topo = w.topo;
-			valid = 0;
-		}
-		C2T<T> a{T(0), T(0)};
-		for (int t = w.term0; t < w.term1; ++t) {
-			const SymTerm st = P.terms[t];
-			if (!((valid >> st.perm) & 1u)) {
-				const int32_t* perm = P.perms + 3 * st.perm;
-				LV g[3];
-				if (P.masses[perm[0]] == P.masses[0] && P.masses[perm[1]] == P.masses[1] &&
-				    P.masses[perm[2]] == P.masses[2]) {
-					for (int i = 0; i < 3; ++i)
-						g[i] = g0[perm[i]];
-				} else {
-					gjFrame(P, bp, fp, perm, g);
+	const Coef4<T> k = coefAt<T>(P, d.coef0);
+	T r = k.c[0];
+	if (d.n > 1) {
+		r = r * c2 + k.c[1] * s2;
+		if (d.n > 2) {
+			T sk = s2 * s2;
+			r = r * c2 + k.c[2] * sk;
+			if (d.n > 3) {
+				sk *= s2;
+				r = r * c2 + k.c[3] * sk;
+				for (int i = 4; i < d.n; ++i) {
+					sk *= s2;
+					r = r * c2 + coefAt<T>(P, d.coef0 + (i & ~3)).c[i & 3] * sk;
 				}
-				kin[st.perm] = kinematics<T>(g, w, P.canonical != 0);
-				valid |= 1u << st.perm;
 			}
-			a = cadd(a, cscale(termAmplitude<T>(P, w, kin[st.perm]), pick<T>(st.factor, st.factorF)));
 		}
-		out[2 * ((uint64_t)wi * ld + e)] = a.re;
-		out[2 * ((uint64_t)wi * ld + e) + 1] = a.im;
+	}
+	return r * (t.get(B.atC + d.c) * t.get(B.atS + d.s));
+}
+
+// the entries that depend on the kinematics alone
+template <typename T>
+PWA_HD void fillTable(const PlanView& P, const Batch& B, const Kin<T>& k, const Table<T>& t)
+{
+	t.powers(B.atC, k.cI, B.pow);
+	t.powers(B.atS, k.sI, B.pow);
+	for (int i = B.e0; i < B.e1; ++i) {
+		const EOp& op = P.eops[i];
+		C2T<T> e = cpowi(k.uH, op.lam);
+		if (P.canonical)
+			e = cmul(e, cpowi(k.u, -op.lam));
+		t.setc(B.atE + 2 * (i - B.e0), cscale(e, dValue<T>(P, B, op.d, t, k.c2I, k.s2I)));
+	}
+	for (int i = B.iso0; i < B.iso1; ++i) {
+		const WaveDev& w = P.waves[P.isoWave[i]];
+		const C2T<T> md = massDependence<T>(P, w, k.mI, deltaM2(w, k), k.mId);
+		t.setc(B.atIso + 2 * (i - B.iso0), cscale(md, static_cast<T>(sqrt(barrierF2<T>(P, w.LI, k.qI)))));
+	}
+	for (int i = B.phase0; i < B.phase1; ++i)
+		t.setc(B.atPhase + 2 * (i - B.phase0), cpowi(k.u, P.phaseM[i]));
+	for (int i = B.lx0; i < B.lx1; ++i)
+		t.set(B.atLx + i - B.lx0, static_cast<T>(sqrt(barrierF2<T>(P, P.lxL[i], k.qX))));
+	t.powers(B.atC, k.cX, B.pow);
+	t.powers(B.atS, k.sX, B.pow);
+}
+
+// the waves of a batch from the table: emit(WaveOp, amplitude without the
+// symmetrisation factor)
+template <typename T, typename Emit>
+PWA_HD void batchWaves(const PlanView& P, const Batch& B, const Table<T>& t, T c2, T s2, Emit emit)
+{
+	int w = B.wave0;
+	for (int f = B.fam0; f < B.fam1; ++f) {
+		const FamOp F = P.fams[f];
+		for (int i = F.d0; i < F.d1; ++i)
+			t.set(B.atD + i - F.d0, dValue<T>(P, B, P.dops[i], t, c2, s2));
+		for (int i = F.x0; i < F.x1; ++i) {
+			const XOp<T> X = xopAt<T>(P, i);
+			const T p = X.a * t.get(X.dP), m = X.r * t.get(X.dM);
+			C2T<T> v{p + m, T(0)};
+			if (X.phase >= 0) {
+				const C2T<T> u = t.getc(X.phase);
+				v = C2T<T>{v.re * u.re, (p - m) * (X.negM ? -u.im : u.im)};
+			}
+			t.setc(B.atX + 2 * (i - F.x0), v);
+		}
+		for (int i = F.ang0; i < F.ang1; ++i) {
+			const AngOp A = P.angs[i];
+			C2T<T> v{T(0), T(0)};
+			int l = A.lam0;
+			// two at a time: the loads of both are in flight together
+			for (; l + 1 < A.lam1; l += 2) {
+				const LamOp<T> L = lamAt<T>(P, l), N = lamAt<T>(P, l + 1);
+				v = cadd(v, cadd(cmul(cscale(t.getc(L.x), L.coef), t.getc(L.e)),
+				                 cmul(cscale(t.getc(N.x), N.coef), t.getc(N.e))));
+			}
+			if (l < A.lam1) {
+				const LamOp<T> L = lamAt<T>(P, l);
+				v = cadd(v, cmul(cscale(t.getc(L.x), L.coef), t.getc(L.e)));
+			}
+			v = cscale(v, t.get(A.lx));
+			for (; w < A.wave1; ++w) {
+				const WaveOp W = P.waveOps[w];
+				emit(W, cmul(v, t.getc(W.iso)));
+			}
+		}
 	}
 }
+
+// the four-vectors of instance permutation `perm`: a permutation that only
+// exchanges particles of equal mass permutes those of the event
+PWA_HD bool permutesEqualMasses(const PlanView& P, const int32_t* perm)
+{
+	return P.masses[perm[0]] == P.masses[0] && P.masses[perm[1]] == P.masses[1] && P.masses[perm[2]] == P.masses[2];
+}
+
+#if !defined(__CUDA_ARCH__)
+// all waves of one event on the host, the kernel's arithmetic one instance
+// after the other; out is complex [wave][ld] as interleaved T (complex128 for
+// T = double, complex64 for T = float: FP64 frames and kinematics, per-wave
+// arithmetic in T)
+template <typename T>
+inline void eventAmplitudes(const PlanView& P, const double bp[3], const double fp[3][3], T* out, uint64_t ld,
+                            uint64_t e)
+{
+	C2T<T>* const pairs = new C2T<T>[(P.tableSize + 1) / 2];
+	T* const tab = &pairs[0].re;
+	for (uint32_t w = 0; w < P.nWaves; ++w)
+		out[2 * ((uint64_t)w * ld + e)] = out[2 * ((uint64_t)w * ld + e) + 1] = T(0);
+	for (uint32_t b = 0; b < P.nBatches; ++b) {
+		const Batch& B = P.batches[b];
+		for (int i = 0; i < B.nInst; ++i) {
+			const int32_t* perm = P.perms + 3 * P.insts[B.inst0 + i];
+			double q[3][3];
+			for (int j = 0; j < 9; ++j)
+				q[j / 3][j % 3] = fp[perm[j / 3]][j % 3];
+			LV g[3];
+			gjFrame(P, bp, q, g);
+			const Kin<T> k = kinematics<T>(g[B.a], g[B.b], g[B.c], B.bachelorFirst != 0, P.canonical != 0);
+			const Table<T> t{tab, 1};
+			fillTable<T>(P, B, k, t);
+			batchWaves<T>(P, B, t, k.c2X, k.s2X, [&](const WaveOp& W, C2T<T> v) {
+				const T f = pick<T>(P.factors[W.factor0 + i], P.factorsF[W.factor0 + i]);
+				if (f == T(0))
+					return;
+				out[2 * ((uint64_t)W.wave * ld + e)] += f * v.re;
+				out[2 * ((uint64_t)W.wave * ld + e) + 1] += f * v.im;
+			});
+		}
+	}
+	delete[] pairs;
+}
+#endif
 
 }  // namespace iso
 }  // namespace pwa

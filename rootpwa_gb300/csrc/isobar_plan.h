@@ -14,7 +14,7 @@
 #include <cmath>
 #include <cstdint>
 #include <string>
-#include <tuple>
+#include <utility>
 #include <vector>
 
 namespace pwa {
@@ -135,17 +135,56 @@ inline std::string checkWave(const pwa_isobar_wave& w, bool reflBasis)
 	return std::string();
 }
 
+// one spin projection of the isobar in one wave: the X-vertex angular part
+// cPlus e^{i M phi/2} dPlus(theta) + cMinus e^{-i M phi/2} dMinus(theta)
+// (couplings, norms and the reflectivity combination folded into cPlus,
+// cMinus) times the isobar vertex e^{i lamIso phiH/2} dIso(thetaH).
+// Helicity formalism: dPlus/dMinus = d^J_{+-M lam}, dIso = d^j_{lam 0}.
+// Canonical formalism: dPlus/dMinus = d^L_{+-M-m, 0} (spherical harmonics
+// Y_L), dIso = d^l_{m 0}, and the whole times e^{-i m phi/2}.
+struct LamTerm {
+	int32_t lamIso;                 // 2 lambda (helicity) or 2 m (canonical) of the isobar
+	std::vector<DTerm> plus, minus, iso;  // minus empty if unused
+	double cPlus, cMinus;
+};
+
+// a permutation of the three final-state slots: slot i takes particle p[i]
+typedef std::vector<int> Perm;
+struct Term {
+	Perm perm;
+	double factor;
+};
+
+// a wave as buildPlan collects it, before compilePlan
+struct WaveSource {
+	int32_t J, M;
+	std::vector<LamTerm> lams;
+	std::vector<std::pair<int, double>> terms;  // (permutation index, factor)
+	int32_t iso;                    // first wave of its isobar class
+};
+
 struct Plan {
 	std::vector<WaveDev> waves;
-	std::vector<int32_t> order;
-	std::vector<LamTerm> lams;
-	std::vector<DTerm> dterms;
-	double bfPoly[8][8];
+	std::vector<WaveSource> source;
+	std::vector<Batch> batches;
+	std::vector<int32_t> insts, isoWave, phaseM, lxL;
+	std::vector<EOp> eops;
+	std::vector<FamOp> fams;
+	std::vector<DOp> dops;
+	std::vector<double> coef, factors;
+	std::vector<float> coefF, factorsF;
+	std::vector<AngOp> angs;
+	std::vector<XOp<double>> xops;
+	std::vector<XOp<float>> xopsF;
+	std::vector<LamOp<double>> lams;
+	std::vector<LamOp<float>> lamsF;
+	std::vector<WaveOp> waveOps;
+	alignas(16) double bfPoly[8][8];
 	double bfNorm[8];
-	float bfPolyF[8][8];            // FP32 copies (complex64 mode)
+	alignas(16) float bfPolyF[8][8];            // FP32 copies (complex64 mode)
 	float bfNormF[8];
 	std::vector<int32_t> perms;     // the six permutations of three slots
-	std::vector<SymTerm> terms;
+	int32_t maxInst = 1, tableSize = 0;
 	double masses[3] = {0.0, 0.0, 0.0}, beamMass = 0.0;
 	int32_t spaceInversion = 0, reflection = 0, canonical = 0;
 
@@ -153,16 +192,33 @@ struct Plan {
 	{
 		PlanView v{};
 		v.waves = waves.data();
-		v.order = order.data();
+		v.batches = batches.data();
+		v.insts = insts.data();
+		v.eops = eops.data();
+		v.isoWave = isoWave.data();
+		v.phaseM = phaseM.data();
+		v.lxL = lxL.data();
+		v.fams = fams.data();
+		v.dops = dops.data();
+		v.coef = coef.data();
+		v.coefF = coefF.data();
+		v.angs = angs.data();
+		v.xops = xops.data();
+		v.xopsF = xopsF.data();
 		v.lams = lams.data();
-		v.dterms = dterms.data();
+		v.lamsF = lamsF.data();
+		v.waveOps = waveOps.data();
+		v.factors = factors.data();
+		v.factorsF = factorsF.data();
 		v.bfPoly = &bfPoly[0][0];
 		v.bfNorm = bfNorm;
 		v.bfPolyF = &bfPolyF[0][0];
 		v.bfNormF = bfNormF;
 		v.perms = perms.data();
-		v.terms = terms.data();
 		v.nWaves = (uint32_t)waves.size();
+		v.nBatches = (uint32_t)batches.size();
+		v.maxInst = maxInst;
+		v.tableSize = tableSize;
 		for (int i = 0; i < 3; ++i)
 			v.masses[i] = masses[i];
 		v.beamMass = beamMass;
@@ -179,14 +235,14 @@ struct Plan {
 // denominators takes M as an FP32 hi + lo pair
 inline void fillFp32Copies(Plan& plan)
 {
-	for (DTerm& t : plan.dterms)
-		t.coefF = (float)t.coef;
-	for (LamTerm& t : plan.lams) {
-		t.cPlusF = (float)t.cPlus;
-		t.cMinusF = (float)t.cMinus;
-	}
-	for (SymTerm& t : plan.terms)
-		t.factorF = (float)t.factor;
+	plan.coefF.assign(plan.coef.begin(), plan.coef.end());
+	plan.factorsF.assign(plan.factors.begin(), plan.factors.end());
+	plan.lamsF.clear();
+	for (const LamOp<double>& l : plan.lams)
+		plan.lamsF.push_back(LamOp<float>{(float)l.coef, l.x, l.e});
+	plan.xopsF.clear();
+	for (const XOp<double>& x : plan.xops)
+		plan.xopsF.push_back(XOp<float>{(float)x.a, (float)x.r, x.dP, x.dM, x.phase, x.negM});
 	for (int i = 0; i < 8; ++i) {
 		for (int k = 0; k < 8; ++k)
 			plan.bfPolyF[i][k] = (float)plan.bfPoly[i][k];
@@ -197,7 +253,8 @@ inline void fillFp32Copies(Plan& plan)
 		w.m0F = (float)w.m0;
 		w.g0F = (float)w.g0;
 		w.q0F = (float)w.q0;
-		w.f2q0F = (float)w.f2q0;
+		w.kG = w.q0 > 0.0 ? w.g0 * w.m0 * w.m0 / (w.q0 * w.f2q0) : 0.0;
+		w.kGF = (float)w.kG;
 		w.maF = (float)w.ma;
 		w.mbF = (float)w.mb;
 		w.q02F = (float)w.q02;
@@ -207,11 +264,360 @@ inline void fillFp32Copies(Plan& plan)
 	}
 }
 
-// a permutation of the three final-state slots: slot i takes particle p[i]
-typedef std::vector<int> Perm;
-struct Term {
-	Perm perm;
-	double factor;
+// Table entries a batch may take: 640 FP64 entries for the 32 threads of the
+// smallest block are 160 KiB of shared memory.
+constexpr int kMaxTable = 640;
+
+// Compiles the collected waves into batches (isobar_math.cuh).  The waves of
+// one topology class are taken family by family -- helicity formalism: equal
+// J and |M|; canonical: equal X-vertex L -- and within a family by angular
+// sum; a batch is closed when the next wave's entries would not fit.
+class PlanCompiler {
+public:
+	explicit PlanCompiler(Plan& p) : P(p) {}
+
+	void run()
+	{
+		P.batches.clear();
+		P.insts.clear();
+		P.isoWave.clear();
+		P.phaseM.clear();
+		P.lxL.clear();
+		P.eops.clear();
+		P.fams.clear();
+		P.dops.clear();
+		P.coef.clear();
+		P.factors.clear();
+		P.angs.clear();
+		P.lams.clear();
+		P.xops.clear();
+		P.waveOps.clear();
+		P.maxInst = 1;
+		P.tableSize = 1;
+		std::vector<int> left(P.waves.size());
+		for (size_t i = 0; i < left.size(); ++i)
+			left[i] = (int)i;
+		while (!left.empty()) {
+			const WaveDev& first = P.waves[left[0]];
+			std::vector<int> mine, others;
+			for (int w : left)
+				(sameTopology(P.waves[w], first) ? mine : others).push_back(w);
+			left.swap(others);
+			topology(mine);
+		}
+	}
+
+private:
+	Plan& P;
+	// batch under construction
+	struct Ang {
+		int L;
+		std::vector<LamOp<double>> lams;
+		std::vector<int> waves;
+	};
+	struct Fam {
+		std::pair<int, int> key;
+		std::vector<std::vector<DTerm>> ds;
+		std::vector<XOp<double>> xs;  // phase: 2M
+		std::vector<Ang> angs;
+	};
+	struct Draft {
+		std::vector<int> insts, isos, phases, ls;
+		std::vector<std::pair<int, std::vector<DTerm>>> es;  // (2 lam, d function)
+		std::vector<Fam> fams;
+		int pow = 0;
+		int size() const
+		{
+			return (int)(2 * (pow + 1) + 2 * (es.size() + isos.size() + phases.size() + mostX()) + ls.size() + mostD());
+		}
+		size_t mostX() const
+		{
+			size_t n = 0;
+			for (const Fam& f : fams)
+				n = std::max(n, f.xs.size());
+			return n;
+		}
+		size_t mostD() const
+		{
+			size_t n = 0;
+			for (const Fam& f : fams)
+				n = std::max(n, f.ds.size());
+			return n;
+		}
+	};
+
+	static bool sameTopology(const WaveDev& x, const WaveDev& y)
+	{
+		return x.a == y.a && x.b == y.b && x.c == y.c && x.bachelorFirst == y.bachelorFirst;
+	}
+	std::pair<int, int> family(int w) const
+	{
+		if (P.canonical)
+			return std::make_pair((int)P.waves[w].LX, 0);
+		return std::make_pair((int)P.source[w].J, std::abs(P.source[w].M));
+	}
+	static int find(std::vector<int>& v, int x)
+	{
+		const size_t i = std::find(v.begin(), v.end(), x) - v.begin();
+		if (i == v.size())
+			v.push_back(x);
+		return (int)i;
+	}
+	// +1 or -1 when y is x or -x term by term, else 0 (the same function from
+	// another formula may differ in the last bits of its coefficients)
+	static int sameD(const std::vector<DTerm>& x, const std::vector<DTerm>& y)
+	{
+		if (x.size() != y.size())
+			return 0;
+		int s = 0;
+		for (size_t i = 0; i < x.size(); ++i) {
+			if (x[i].a != y[i].a || x[i].b != y[i].b)
+				return 0;
+			const int si = std::fabs(x[i].coef - y[i].coef) <= 1e-14 * std::fabs(x[i].coef)   ? 1
+			               : std::fabs(x[i].coef + y[i].coef) <= 1e-14 * std::fabs(x[i].coef) ? -1
+			                                                                                  : 0;
+			if (si == 0 || (s != 0 && si != s))
+				return 0;
+			s = si;
+		}
+		return s;
+	}
+	static int powerOf(const std::vector<DTerm>& t)
+	{
+		int p = 0;
+		for (const DTerm& d : t)
+			p = std::max(p, std::max(d.a, d.b));
+		return p;
+	}
+	// entry of the d function in its family, and the sign it comes with
+	static int findD(Fam& f, const std::vector<DTerm>& t, double* sign)
+	{
+		for (size_t i = 0; i < f.ds.size(); ++i) {
+			const int s = sameD(f.ds[i], t);
+			if (s != 0) {
+				*sign = s;
+				return (int)i;
+			}
+		}
+		f.ds.push_back(t);
+		*sign = 1.0;
+		return (int)f.ds.size() - 1;
+	}
+	// entry of the X-vertex sum (of equal ratio up to rounding)
+	static int findX(Fam& f, const XOp<double>& x)
+	{
+		for (size_t i = 0; i < f.xs.size(); ++i) {
+			const XOp<double>& y = f.xs[i];
+			if (y.a == x.a && std::fabs(y.r - x.r) <= 1e-14 * std::fabs(x.r) && y.dP == x.dP && y.dM == x.dM &&
+			    y.phase == x.phase)
+				return (int)i;
+		}
+		f.xs.push_back(x);
+		return (int)f.xs.size() - 1;
+	}
+	int findE(Draft& d, int lam, const std::vector<DTerm>& t) const
+	{
+		for (size_t i = 0; i < d.es.size(); ++i)
+			if (d.es[i].first == lam && sameD(d.es[i].second, t) == 1)
+				return (int)i;
+		d.es.push_back(std::make_pair(lam, t));
+		return (int)d.es.size() - 1;
+	}
+
+	void add(Draft& d, int w) const
+	{
+		const WaveSource& src = P.source[w];
+		for (const auto& t : src.terms)
+			find(d.insts, t.first);
+		find(d.isos, src.iso);
+		find(d.ls, P.waves[w].LX);
+		if (src.M != 0)
+			find(d.phases, std::abs(src.M));
+		const std::pair<int, int> key = family(w);
+		Fam* f = nullptr;
+		for (Fam& x : d.fams)
+			if (x.key == key)
+				f = &x;
+		if (!f) {
+			d.fams.push_back(Fam());
+			f = &d.fams.back();
+			f->key = key;
+		}
+		Ang a;
+		a.L = P.waves[w].LX;
+		for (const LamTerm& l : src.lams) {
+			XOp<double> x{};
+			LamOp<double> op{};
+			double cP = 0.0, cM = 0.0, s = 1.0;
+			if (!l.plus.empty()) {
+				x.dP = findD(*f, l.plus, &s);
+				cP = s * l.cPlus;
+				d.pow = std::max(d.pow, powerOf(l.plus));
+			}
+			if (!l.minus.empty()) {
+				x.dM = findD(*f, l.minus, &s);
+				cM = s * l.cMinus;
+				d.pow = std::max(d.pow, powerOf(l.minus));
+			}
+			if (l.plus.empty())
+				x.dP = x.dM;
+			if (l.minus.empty())
+				x.dM = x.dP;
+			x.phase = src.M;
+			x.a = cP != 0.0 ? 1.0 : 0.0;
+			x.r = cP != 0.0 ? cM / cP : 1.0;
+			op.coef = cP != 0.0 ? cP : cM;
+			op.x = findX(*f, x);
+			op.e = findE(d, l.lamIso, l.iso);
+			d.pow = std::max(d.pow, powerOf(l.iso));
+			a.lams.push_back(op);
+		}
+		auto sameLams = [](const std::vector<LamOp<double>>& x, const std::vector<LamOp<double>>& y) {
+			return std::equal(x.begin(), x.end(), y.begin(), y.end(), [](const LamOp<double>& p, const LamOp<double>& q) {
+				return p.x == q.x && p.e == q.e && p.coef == q.coef;
+			});
+		};
+		for (Ang& x : f->angs)
+			if (x.L == a.L && sameLams(x.lams, a.lams)) {
+				x.waves.push_back(w);
+				return;
+			}
+		a.waves.push_back(w);
+		f->angs.push_back(a);
+	}
+
+	void topology(std::vector<int> waves)
+	{
+		std::stable_sort(waves.begin(), waves.end(), [&](int x, int y) { return family(x) < family(y); });
+		Draft d;
+		bool any = false;
+		for (int w : waves) {
+			Draft next = d;
+			add(next, w);
+			if (any && next.size() > kMaxTable) {
+				emit(d);
+				next = Draft();
+				add(next, w);
+			}
+			d = next;
+			any = true;
+		}
+		emit(d);
+	}
+
+	DOp dop(const std::vector<DTerm>& t)
+	{
+		DOp o{};
+		o.coef0 = (int32_t)P.coef.size();
+		o.n = (int32_t)t.size();
+		o.c = t.back().a;
+		o.s = t.front().b;
+		for (const DTerm& x : t)
+			P.coef.push_back(x.coef);
+		P.coef.resize((P.coef.size() + 3) / 4 * 4, 0.0);
+		return o;
+	}
+
+	void emit(const Draft& d)
+	{
+		Batch B{};
+		const WaveDev& w0 = P.waves[d.fams[0].angs[0].waves[0]];
+		B.a = w0.a;
+		B.b = w0.b;
+		B.c = w0.c;
+		B.bachelorFirst = w0.bachelorFirst;
+		B.inst0 = (int32_t)P.insts.size();
+		B.nInst = (int32_t)d.insts.size();
+		P.insts.insert(P.insts.end(), d.insts.begin(), d.insts.end());
+		B.pow = d.pow;
+		int at = 0;
+		B.atE = at;
+		B.atIso = (at += 2 * (int)d.es.size());
+		B.atPhase = (at += 2 * (int)d.isos.size());
+		B.atX = (at += 2 * (int)d.phases.size());
+		B.atC = (at += 2 * (int)d.mostX());
+		B.atS = (at += d.pow + 1);
+		B.atLx = (at += d.pow + 1);
+		B.atD = (at += (int)d.ls.size());
+		B.e0 = (int32_t)P.eops.size();
+		for (const auto& e : d.es) {
+			EOp op{};
+			op.d = dop(e.second);
+			op.lam = e.first;
+			P.eops.push_back(op);
+		}
+		B.e1 = (int32_t)P.eops.size();
+		auto put = [](std::vector<int32_t>& to, const std::vector<int>& v, int32_t* i0, int32_t* i1) {
+			*i0 = (int32_t)to.size();
+			to.insert(to.end(), v.begin(), v.end());
+			*i1 = (int32_t)to.size();
+		};
+		put(P.isoWave, d.isos, &B.iso0, &B.iso1);
+		put(P.phaseM, d.phases, &B.phase0, &B.phase1);
+		put(P.lxL, d.ls, &B.lx0, &B.lx1);
+		auto where = [](const std::vector<int>& v, int x) {
+			return (int)(std::find(v.begin(), v.end(), x) - v.begin());
+		};
+		const size_t factors0 = P.factors.size();
+		B.fam0 = (int32_t)P.fams.size();
+		B.wave0 = (int32_t)P.waveOps.size();
+		for (const Fam& f : d.fams) {
+			FamOp F{};
+			F.d0 = (int32_t)P.dops.size();
+			for (const auto& t : f.ds)
+				P.dops.push_back(dop(t));
+			F.d1 = (int32_t)P.dops.size();
+			F.x0 = (int32_t)P.xops.size();
+			for (XOp<double> x : f.xs) {
+				const int M = x.phase;
+				x.dP += B.atD;
+				x.dM += B.atD;
+				x.phase = M == 0 ? -1 : B.atPhase + 2 * where(d.phases, std::abs(M));
+				x.negM = M < 0 ? 1 : 0;
+				P.xops.push_back(x);
+			}
+			F.x1 = (int32_t)P.xops.size();
+			F.ang0 = (int32_t)P.angs.size();
+			for (const Ang& a : f.angs) {
+				AngOp A{};
+				A.lam0 = (int32_t)P.lams.size();
+				for (LamOp<double> l : a.lams) {
+					l.x = B.atX + 2 * l.x;
+					l.e = B.atE + 2 * l.e;
+					P.lams.push_back(l);
+				}
+				A.lam1 = (int32_t)P.lams.size();
+				A.lx = B.atLx + where(d.ls, a.L);
+				for (int w : a.waves) {
+					WaveOp W{};
+					W.wave = w;
+					W.iso = B.atIso + 2 * where(d.isos, P.source[w].iso);
+					std::vector<double> row(d.insts.size(), 0.0);
+					for (const auto& t : P.source[w].terms)
+						row[where(d.insts, t.first)] += t.second;
+					// waves of equal factors share a row (all of a Bose-symmetrised set)
+					W.factor0 = -1;
+					for (size_t k = factors0; W.factor0 < 0 && k + row.size() <= P.factors.size() && !row.empty();
+					     k += row.size())
+						if (std::equal(row.begin(), row.end(), P.factors.begin() + k))
+							W.factor0 = (int32_t)k;
+					if (W.factor0 < 0) {
+						W.factor0 = (int32_t)P.factors.size();
+						P.factors.insert(P.factors.end(), row.begin(), row.end());
+					}
+					P.waveOps.push_back(W);
+				}
+				A.wave1 = (int32_t)P.waveOps.size();
+				P.angs.push_back(A);
+			}
+			F.ang1 = (int32_t)P.angs.size();
+			P.fams.push_back(F);
+		}
+		B.fam1 = (int32_t)P.fams.size();
+		P.batches.push_back(B);
+		P.maxInst = std::max(P.maxInst, B.nInst);
+		P.tableSize = std::max(P.tableSize, (int32_t)d.size());
+	}
 };
 
 // index of a permutation in the lexicographic list of the six (the kernel's table)
@@ -383,7 +789,7 @@ inline std::vector<Term> symTerms(const pwa_isobar_wave& w, const int32_t specie
 // isobar vertex sqrt(4 pi) (0 0 0 0 | S' 0) F_l (l m S' 0 | j m) Y_l^m.  The
 // (L mL S m | J +-M) couplings vanish unless mL = +-M - m, so the sum over mL
 // keeps two terms; sqrt(4 pi) Y_L^mu = sqrt(2L+1) e^{i mu phi} d^L_{mu 0}.
-inline void addCanonicalTerms(const pwa_isobar_wave& s, bool reflBasis, Plan& plan)
+inline void addCanonicalTerms(const pwa_isobar_wave& s, bool reflBasis, std::vector<LamTerm>& lams)
 {
 	const int J = s.J, M = s.M, L = s.L, S = s.S, j = s.isobarJ, l = s.isobarL, Si = s.isobarS;
 	for (int m = -j; m <= j; m += 2) {
@@ -416,22 +822,14 @@ inline void addCanonicalTerms(const pwa_isobar_wave& s, bool reflBasis, Plan& pl
 		const double c = std::sqrt(L + 1.0) * ss * iso;
 		LamTerm t{};
 		t.lamIso = m;
-		t.plus0 = (int32_t)plan.dterms.size();
 		if (cP != 0.0)
-			wignerTerms(L, mP, 0, plan.dterms);
-		t.plus1 = (int32_t)plan.dterms.size();
-		t.minus0 = t.plus1;
+			wignerTerms(L, mP, 0, t.plus);
 		if (cM != 0.0)
-			wignerTerms(L, mM, 0, plan.dterms);
-		t.minus1 = (int32_t)plan.dterms.size();
-		t.iso0 = t.minus1;
-		wignerTerms(l, m, 0, plan.dterms);
-		t.iso1 = (int32_t)plan.dterms.size();
-		t.mPlus = mP;
-		t.mMinus = mM;
+			wignerTerms(L, mM, 0, t.minus);
+		wignerTerms(l, m, 0, t.iso);
 		t.cPlus = c * cP;
 		t.cMinus = c * cM;
-		plan.lams.push_back(t);
+		lams.push_back(t);
 	}
 }
 
@@ -455,9 +853,7 @@ inline std::string buildPlan(const std::vector<pwa_isobar_wave>& specs, const do
 	plan.spaceInversion = spaceInversion ? 1 : 0;
 	plan.reflection = reflection ? 1 : 0;
 	plan.waves.clear();
-	plan.lams.clear();
-	plan.dterms.clear();
-	plan.terms.clear();
+	plan.source.clear();
 	barrierPolynomials(plan.bfPoly, plan.bfNorm);
 	plan.perms.clear();
 	{
@@ -466,14 +862,15 @@ inline std::string buildPlan(const std::vector<pwa_isobar_wave>& specs, const do
 			plan.perms.insert(plan.perms.end(), q, q + 3);
 		while (std::next_permutation(q, q + 3));
 	}
-	std::vector<std::tuple<int, int, int, int>> topoKeys;
 	for (const pwa_isobar_wave& s : specs) {
 		WaveDev w{};
+		WaveSource src{};
+		src.J = s.J;
+		src.M = s.M;
 		w.a = s.isobarDaughter1;
 		w.b = s.isobarDaughter2;
 		w.c = s.bachelor;
 		w.bachelorFirst = s.bachelorFirst ? 1 : 0;
-		w.M = s.M;
 		w.LX = s.L;
 		w.LI = s.isobarL;
 		w.massDep = s.massDependence;
@@ -484,7 +881,7 @@ inline std::string buildPlan(const std::vector<pwa_isobar_wave>& specs, const do
 		w.f2q0 = 1.0;
 		for (int k = 0; k < 10; ++k)
 			w.mdp[k] = s.massDepParams[k];
-		w.q02 = breakup2(s.isobarMass, w.ma, w.mb);
+		w.q02 = s.isobarMass > 0 ? breakup2(s.isobarMass, w.ma, w.mb) : 0.0;  // not NaN: it is compared below
 		if (s.massDependence == kMassRelBw) {
 			// the PWA2000 rule q0 = sqrt|q0^2| (massDependence.cc:268-270)
 			w.q0 = std::sqrt(std::fabs(w.q02));
@@ -497,16 +894,9 @@ inline std::string buildPlan(const std::vector<pwa_isobar_wave>& specs, const do
 				       ": the isobar mass is below the threshold of its daughters";
 			w.q0 = std::sqrt(w.q02);
 		}
-		w.term0 = (int32_t)plan.terms.size();
 		for (const Term& t : symTerms(s, species, bose, isospin))
 			if (t.factor != 0.0)  // zero terms (a vanishing isospin coupling) only enter the normalisation
-				plan.terms.push_back(SymTerm{permIndex(t.perm), 0.f, t.factor});
-		w.term1 = (int32_t)plan.terms.size();
-		const std::tuple<int, int, int, int> key(w.a, w.b, w.c, w.bachelorFirst);
-		auto it = std::find(topoKeys.begin(), topoKeys.end(), key);
-		w.topo = (int32_t)(it - topoKeys.begin());
-		if (it == topoKeys.end())
-			topoKeys.push_back(key);
+				src.terms.push_back(std::make_pair(permIndex(t.perm), t.factor));
 		// reflectivity combination of the X vertex
 		double wPlus = 1.0, wMinus = 0.0;
 		bool zero = false;
@@ -519,14 +909,9 @@ inline std::string buildPlan(const std::vector<pwa_isobar_wave>& specs, const do
 				wMinus = -f / std::sqrt(2.0);
 			}
 		}
-		w.lam0 = (int32_t)plan.lams.size();
-		if (canonical) {
-			addCanonicalTerms(s, reflBasis, plan);
-			w.lam1 = (int32_t)plan.lams.size();
-			plan.waves.push_back(w);
-			continue;
-		}
-		for (int lamIso = -s.isobarJ; lamIso <= s.isobarJ && !zero; lamIso += 2) {
+		if (canonical)
+			addCanonicalTerms(s, reflBasis, src.lams);
+		for (int lamIso = -s.isobarJ; lamIso <= s.isobarJ && !zero && !canonical; lamIso += 2) {
 			// X -> daughter 1 + daughter 2 with helicities (l1, l2), spins (s1, s2)
 			const int s1 = s.bachelorFirst ? 0 : s.isobarJ, l1 = s.bachelorFirst ? 0 : lamIso;
 			const int s2 = s.bachelorFirst ? s.isobarJ : 0, l2 = s.bachelorFirst ? lamIso : 0;
@@ -541,25 +926,16 @@ inline std::string buildPlan(const std::vector<pwa_isobar_wave>& specs, const do
 			const double c = std::sqrt(s.L + 1.0) * cgX * std::sqrt(s.isobarL + 1.0) * cgI;
 			LamTerm t{};
 			t.lamIso = lamIso;
-			t.plus0 = (int32_t)plan.dterms.size();
-			wignerTerms(s.J, s.M, lam, plan.dterms);
-			t.plus1 = (int32_t)plan.dterms.size();
-			t.minus0 = t.minus1 = t.plus1;
-			if (wMinus != 0.0) {
-				wignerTerms(s.J, -s.M, lam, plan.dterms);
-				t.minus1 = (int32_t)plan.dterms.size();
-			}
-			t.iso0 = (int32_t)plan.dterms.size();
-			wignerTerms(s.isobarJ, lamIso, 0, plan.dterms);
-			t.iso1 = (int32_t)plan.dterms.size();
+			wignerTerms(s.J, s.M, lam, t.plus);
+			if (wMinus != 0.0)
+				wignerTerms(s.J, -s.M, lam, t.minus);
+			wignerTerms(s.isobarJ, lamIso, 0, t.iso);
 			t.cPlus = c * wPlus;
 			t.cMinus = c * wMinus;
-			t.mPlus = s.M;
-			t.mMinus = -s.M;
-			plan.lams.push_back(t);
+			src.lams.push_back(t);
 		}
-		w.lam1 = (int32_t)plan.lams.size();
 		plan.waves.push_back(w);
+		plan.source.push_back(src);
 	}
 	// isobar classes: waves whose mass dependence (kind and parameters) and
 	// isobar barrier factor agree share their product per event and term
@@ -573,30 +949,14 @@ inline std::string buildPlan(const std::vector<pwa_isobar_wave>& specs, const do
 		return true;
 	};
 	for (size_t i = 0; i < plan.waves.size(); ++i) {
-		WaveDev& w = plan.waves[i];
-		w.iso = (int32_t)i;
+		plan.source[i].iso = (int32_t)i;
 		for (size_t j = 0; j < i; ++j)
-			if (sameIsobar(plan.waves[j], w)) {
-				w.iso = plan.waves[j].iso;
+			if (sameIsobar(plan.waves[j], plan.waves[i])) {
+				plan.source[i].iso = plan.source[j].iso;
 				break;
 			}
 	}
-	plan.order.resize(plan.waves.size());
-	for (size_t i = 0; i < plan.order.size(); ++i)
-		plan.order[i] = (int32_t)i;
-	// waves of one topology class together (they share the kinematics), within
-	// a class those of one mass dependence and isobar class, then of one X-vertex
-	// L (they share the cached values)
-	std::stable_sort(plan.order.begin(), plan.order.end(), [&](int32_t x, int32_t y) {
-		const WaveDev &a = plan.waves[x], &b = plan.waves[y];
-		if (a.topo != b.topo)
-			return a.topo < b.topo;
-		if (a.massDep != b.massDep)
-			return a.massDep < b.massDep;
-		if (a.iso != b.iso)
-			return a.iso < b.iso;
-		return a.LX < b.LX;
-	});
+	PlanCompiler(plan).run();
 	fillFp32Copies(plan);
 	return std::string();
 }
