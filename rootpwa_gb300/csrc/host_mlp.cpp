@@ -9,6 +9,8 @@
 struct pwa_mlp {
 	int nIn = 0, h1 = 0, h2 = 0, nOut = 0;
 	size_t oW1 = 0, ob1 = 0, oW2 = 0, ob2 = 0, oW3 = 0, ob3 = 0, nPar = 0;
+	int nInP = 0, h1P = 0, h2P = 0, nOutP = 0;  // padded row lengths of the BF16 matrices
+	MlpWeights map{};                           // weights in the padded BF16 copy
 	cudaStream_t stream = nullptr;
 	DevBuf params, grads, adamM, adamV, w16;
 	// per-batch buffers (capacity cap rows)
@@ -38,16 +40,19 @@ int mlpEnsureBatch(pwa_mlp* N, int B)
 		return kOk;
 	const size_t b = (size_t)B;
 	const int hmax = std::max(N->h1, N->h2);
-	PWA_TRY(N->x16.alloc(b * N->nIn * 2, "MLP input"));
-	PWA_TRY(N->h1b.alloc(b * N->h1 * 2, "MLP activations"));
-	PWA_TRY(N->h2b.alloc(b * N->h2 * 2, "MLP activations"));
+	PWA_TRY(N->x16.alloc(b * N->nInP * 2, "MLP input"));
+	PWA_TRY(N->h1b.alloc(b * N->h1P * 2, "MLP activations"));
+	PWA_TRY(N->h2b.alloc(b * N->h2P * 2, "MLP activations"));
 	PWA_TRY(N->y32.alloc(b * N->nOut * 4, "MLP output"));
 	PWA_TRY(N->t32.alloc(b * N->nOut * 4, "MLP targets"));
 	PWA_TRY(N->dy32.alloc(b * N->nOut * 4, "MLP output gradient"));
-	PWA_TRY(N->dy16.alloc(b * N->nOut * 2, "MLP output gradient"));
-	PWA_TRY(N->dh16.alloc(b * N->h2 * 2, "MLP hidden gradient"));
-	PWA_TRY(N->dh1.alloc(b * N->h1 * 2, "MLP hidden gradient"));
+	PWA_TRY(N->dy16.alloc(b * N->nOutP * 2, "MLP output gradient"));
+	PWA_TRY(N->dh16.alloc(b * N->h2P * 2, "MLP hidden gradient"));
+	PWA_TRY(N->dh1.alloc(b * N->h1P * 2, "MLP hidden gradient"));
 	PWA_TRY(N->dh32.alloc(b * hmax * 4, "MLP hidden gradient"));
+	// the rows' padding stays zero
+	for (DevBuf* p : {&N->x16, &N->h1b, &N->h2b, &N->dy16, &N->dh16, &N->dh1})
+		PWA_TRY(cudaCheck(cudaMemsetAsync(p->p, 0, p->bytes, N->stream), "memset"));
 	PWA_TRY(N->idx.alloc(b * 4, "MLP batch index"));
 	PWA_TRY(N->loss.alloc(sizeof(double), "MLP loss"));
 	N->cap = B;
@@ -60,7 +65,7 @@ int mlpEnsureBatch(pwa_mlp* N, int B)
 int mlpGemm(pwa_mlp* N, MlpGemm g, cudaStream_t s)
 {
 	g.splitK = mlpGemmSplit(g, N->numSMs);
-	const size_t need = (size_t)g.splitK * g.M * g.N;
+	const size_t need = (size_t)g.splitK * g.M * mlpWorkLd(g.N);
 	if (need > N->workFloats) {
 		PWA_TRY(N->work.alloc(need * sizeof(float), "MLP K-slice workspace"));
 		N->workFloats = need;
@@ -84,18 +89,18 @@ int mlpCheckDevice(pwa_mlp* N)
 
 MlpGemm gemmXWt(int M, int N, int K, const uint16_t* X, const uint16_t* W)
 {
-	// C[m][n] = sum_k X[m][k] W[n][k]
+	// C[m][n] = sum_k X[m][k] W[n][k], rows of mlpPad(K) elements
 	MlpGemm g{};
 	g.M = M;
 	g.N = N;
 	g.K = K;
 	g.A = X;
-	g.lda_m = (size_t)K;
+	g.lda_m = (size_t)mlpPad(K);
 	g.lda_k = 1;
 	g.aContigK = 1;
 	g.B = W;
 	g.ldb_k = 1;
-	g.ldb_n = (size_t)K;
+	g.ldb_n = (size_t)mlpPad(K);
 	g.bContigK = 1;
 	return g;
 }
@@ -105,32 +110,34 @@ int mlpForward(pwa_mlp* N, int B)
 {
 	const float* P = N->params.as<float>();
 	const uint16_t* W = N->w16.as<uint16_t>();
-	MlpGemm g = gemmXWt(B, N->h1, N->nIn, N->x16.as<uint16_t>(), W + N->oW1);
+	MlpGemm g = gemmXWt(B, N->h1, N->nIn, N->x16.as<uint16_t>(), W + N->map.to[0]);
 	g.bias = P + N->ob1;
 	g.relu = 1;
 	g.C16 = N->h1b.as<uint16_t>();
+	g.ld16 = N->h1P;
 	PWA_TRY(mlpGemm(N, g, N->stream));
-	g = gemmXWt(B, N->h2, N->h1, N->h1b.as<uint16_t>(), W + N->oW2);
+	g = gemmXWt(B, N->h2, N->h1, N->h1b.as<uint16_t>(), W + N->map.to[1]);
 	g.bias = P + N->ob2;
 	g.relu = 1;
 	g.C16 = N->h2b.as<uint16_t>();
+	g.ld16 = N->h2P;
 	PWA_TRY(mlpGemm(N, g, N->stream));
-	g = gemmXWt(B, N->nOut, N->h2, N->h2b.as<uint16_t>(), W + N->oW3);
+	g = gemmXWt(B, N->nOut, N->h2, N->h2b.as<uint16_t>(), W + N->map.to[2]);
 	g.bias = P + N->ob3;
 	g.C32 = N->y32.as<float>();
 	return mlpGemm(N, g, N->stream);
 }
 
-// gradient of the mean squared error of the batch (targets in t32) into grads
-int mlpBackward(pwa_mlp* N, int B)
+// gradient of the mean squared error of the batch (targets in t32) into
+// grads, the error added to *loss
+int mlpBackward(pwa_mlp* N, int B, double* loss)
 {
 	cudaStream_t s = N->stream;
 	const uint16_t* W = N->w16.as<uint16_t>();
 	float* G = N->grads.as<float>();
-	PWA_TRY(cudaCheck(cudaMemsetAsync(N->loss.p, 0, sizeof(double), s), "memset"));
 	const int nY = B * N->nOut;
-	PWA_TRY(launchMse(N->y32.as<float>(), N->t32.as<float>(), nY, 1.f / (float)nY, N->dy32.as<float>(),
-	                  N->dy16.as<uint16_t>(), N->loss.as<double>(), s));
+	PWA_TRY(launchMse(N->y32.as<float>(), N->t32.as<float>(), nY, N->nOut, N->nOutP, 1.f / (float)nY,
+	                  N->dy32.as<float>(), N->dy16.as<uint16_t>(), loss, s));
 	// dW3[n][k] = sum_b dY[b][n] h2[b][k]
 	MlpGemm g{};
 	g.M = N->nOut;
@@ -138,9 +145,9 @@ int mlpBackward(pwa_mlp* N, int B)
 	g.K = B;
 	g.A = N->dy16.as<uint16_t>();
 	g.lda_m = 1;
-	g.lda_k = (size_t)N->nOut;
+	g.lda_k = (size_t)N->nOutP;
 	g.B = N->h2b.as<uint16_t>();
-	g.ldb_k = (size_t)N->h2;
+	g.ldb_k = (size_t)N->h2P;
 	g.ldb_n = 1;
 	g.C32 = G + N->oW3;
 	PWA_TRY(mlpGemm(N, g, s));
@@ -151,12 +158,13 @@ int mlpBackward(pwa_mlp* N, int B)
 	g.N = N->h2;
 	g.K = N->nOut;
 	g.A = N->dy16.as<uint16_t>();
-	g.lda_m = (size_t)N->nOut;
+	g.lda_m = (size_t)N->nOutP;
 	g.lda_k = 1;
 	g.aContigK = 1;
-	g.B = W + N->oW3;
-	g.ldb_k = (size_t)N->h2;
+	g.B = W + N->map.to[2];
+	g.ldb_k = (size_t)N->h2P;
 	g.ldb_n = 1;
+	g.ld16 = N->h2P;
 	g.mask = N->h2b.as<uint16_t>();
 	g.C16 = N->dh16.as<uint16_t>();
 	g.C32 = N->dh32.as<float>();
@@ -169,9 +177,9 @@ int mlpBackward(pwa_mlp* N, int B)
 	g.K = B;
 	g.A = N->dh16.as<uint16_t>();
 	g.lda_m = 1;
-	g.lda_k = (size_t)N->h2;
+	g.lda_k = (size_t)N->h2P;
 	g.B = N->h1b.as<uint16_t>();
-	g.ldb_k = (size_t)N->h1;
+	g.ldb_k = (size_t)N->h1P;
 	g.ldb_n = 1;
 	g.C32 = G + N->oW2;
 	PWA_TRY(mlpGemm(N, g, s));
@@ -181,12 +189,13 @@ int mlpBackward(pwa_mlp* N, int B)
 	g.N = N->h1;
 	g.K = N->h2;
 	g.A = N->dh16.as<uint16_t>();
-	g.lda_m = (size_t)N->h2;
+	g.lda_m = (size_t)N->h2P;
 	g.lda_k = 1;
 	g.aContigK = 1;
-	g.B = W + N->oW2;
-	g.ldb_k = (size_t)N->h1;
+	g.B = W + N->map.to[1];
+	g.ldb_k = (size_t)N->h1P;
 	g.ldb_n = 1;
+	g.ld16 = N->h1P;
 	g.mask = N->h1b.as<uint16_t>();
 	g.C16 = N->dh1.as<uint16_t>();
 	g.C32 = N->dh32.as<float>();
@@ -199,9 +208,9 @@ int mlpBackward(pwa_mlp* N, int B)
 	g.K = B;
 	g.A = N->dh1.as<uint16_t>();
 	g.lda_m = 1;
-	g.lda_k = (size_t)N->h1;
+	g.lda_k = (size_t)N->h1P;
 	g.B = N->x16.as<uint16_t>();
-	g.ldb_k = (size_t)N->nIn;
+	g.ldb_k = (size_t)N->nInP;
 	g.ldb_n = 1;
 	g.C32 = G + N->oW1;
 	return mlpGemm(N, g, s);
@@ -213,7 +222,7 @@ int mlpAdam(pwa_mlp* N, float lr)
 	++N->step;
 	const float c1 = 1.f - std::pow(b1, (float)N->step), c2 = 1.f - std::pow(b2, (float)N->step);
 	return launchAdam(N->params.as<float>(), N->grads.as<float>(), N->adamM.as<float>(), N->adamV.as<float>(),
-	                  N->w16.as<uint16_t>(), N->nPar, lr, b1, b2, eps, c1, c2, N->stream);
+	                  N->w16.as<uint16_t>(), N->nPar, lr, b1, b2, eps, c1, c2, N->map, N->stream);
 }
 
 int mlpUploadBatch(pwa_mlp* N, const float* X, const float* T, int B)
@@ -223,7 +232,7 @@ int mlpUploadBatch(pwa_mlp* N, const float* X, const float* T, int B)
 	DevBuf x32;
 	PWA_TRY(x32.alloc((size_t)B * N->nIn * 4, "MLP input staging"));
 	PWA_TRY(cudaCheck(cudaMemcpyAsync(x32.p, X, (size_t)B * N->nIn * 4, cudaMemcpyHostToDevice, s), "upload"));
-	PWA_TRY(launchToBf16(x32.as<float>(), N->x16.as<uint16_t>(), (size_t)B * N->nIn, s));
+	PWA_TRY(launchToBf16(x32.as<float>(), N->x16.as<uint16_t>(), (size_t)B, N->nIn, N->nInP, s));
 	if (T)
 		PWA_TRY(cudaCheck(cudaMemcpyAsync(N->t32.p, T, (size_t)B * N->nOut * 4, cudaMemcpyHostToDevice, s), "upload"));
 	return cudaCheck(cudaStreamSynchronize(s), "MLP upload");
@@ -249,13 +258,29 @@ int pwa_mlp_create(pwa_mlp** out, uint32_t nIn, uint32_t nHidden1, uint32_t nHid
 	N->oW3 = N->ob2 + nHidden2;
 	N->ob3 = N->oW3 + (size_t)nOut * nHidden2;
 	N->nPar = N->ob3 + nOut;
+	N->nInP = mlpPad(N->nIn);
+	N->h1P = mlpPad(N->h1);
+	N->h2P = mlpPad(N->h2);
+	N->nOutP = mlpPad(N->nOut);
+	const size_t from[3] = {N->oW1, N->oW2, N->oW3};
+	const int rows[3] = {N->h1, N->h2, N->nOut}, cols[3] = {N->nIn, N->h1, N->h2};
+	size_t to = 0;
+	for (int l = 0; l < 3; ++l) {
+		N->map.from[l] = from[l];
+		N->map.rows[l] = rows[l];
+		N->map.cols[l] = cols[l];
+		N->map.ld[l] = mlpPad(cols[l]);
+		N->map.to[l] = to;
+		to += (size_t)rows[l] * mlpPad(cols[l]);
+	}
 	PWA_TRY(cudaCheck(cudaStreamCreateWithFlags(&N->stream, cudaStreamNonBlocking), "stream"));
 	int dev = 0;
 	PWA_TRY(cudaCheck(cudaGetDevice(&dev), "cudaGetDevice"));
 	PWA_TRY(cudaCheck(cudaDeviceGetAttribute(&N->numSMs, cudaDevAttrMultiProcessorCount, dev), "SM count"));
 	for (DevBuf* b : {&N->params, &N->grads, &N->adamM, &N->adamV})
 		PWA_TRY(b->alloc(N->nPar * 4, "MLP parameters"));
-	PWA_TRY(N->w16.alloc(N->nPar * 2, "MLP BF16 weights"));
+	PWA_TRY(N->w16.alloc(to * 2, "MLP BF16 weights"));
+	PWA_TRY(cudaCheck(cudaMemset(N->w16.p, 0, to * 2), "memset"));
 	PWA_TRY(N->dErr.alloc(sizeof(unsigned), "MLP error flag"));
 	PWA_TRY(cudaCheck(cudaMemset(N->dErr.p, 0, sizeof(unsigned)), "memset"));
 	// He-normal weights (std sqrt(2 / fan_in)), zero biases, from a seeded host RNG
@@ -273,7 +298,7 @@ int pwa_mlp_create(pwa_mlp** out, uint32_t nIn, uint32_t nHidden1, uint32_t nHid
 	PWA_TRY(cudaCheck(cudaMemcpy(N->params.p, p.data(), N->nPar * 4, cudaMemcpyHostToDevice), "upload"));
 	PWA_TRY(cudaCheck(cudaMemset(N->adamM.p, 0, N->nPar * 4), "memset"));
 	PWA_TRY(cudaCheck(cudaMemset(N->adamV.p, 0, N->nPar * 4), "memset"));
-	PWA_TRY(launchToBf16(N->params.as<float>(), N->w16.as<uint16_t>(), N->nPar, N->stream));
+	PWA_TRY(launchWeights16(N->params.as<float>(), N->w16.as<uint16_t>(), N->nPar, N->map, N->stream));
 	PWA_TRY(cudaCheck(cudaStreamSynchronize(N->stream), "MLP init"));
 	*out = N.release();
 	return kOk;
@@ -306,7 +331,7 @@ int pwa_mlp_set_params(pwa_mlp* N, const float* in)
 	if (!N || !in)
 		return setError(kErrArg, "null argument");
 	PWA_TRY(cudaCheck(cudaMemcpyAsync(N->params.p, in, N->nPar * 4, cudaMemcpyHostToDevice, N->stream), "upload"));
-	PWA_TRY(launchToBf16(N->params.as<float>(), N->w16.as<uint16_t>(), N->nPar, N->stream));
+	PWA_TRY(launchWeights16(N->params.as<float>(), N->w16.as<uint16_t>(), N->nPar, N->map, N->stream));
 	PWA_TRY(cudaCheck(cudaMemsetAsync(N->adamM.p, 0, N->nPar * 4, N->stream), "memset"));
 	PWA_TRY(cudaCheck(cudaMemsetAsync(N->adamV.p, 0, N->nPar * 4, N->stream), "memset"));
 	N->step = 0;
@@ -331,7 +356,8 @@ int pwa_mlp_gradient(pwa_mlp* N, const float* X, const float* T, uint32_t B, dou
 		return setError(kErrArg, "null argument or empty batch");
 	PWA_TRY(mlpUploadBatch(N, X, T, (int)B));
 	PWA_TRY(mlpForward(N, (int)B));
-	PWA_TRY(mlpBackward(N, (int)B));
+	PWA_TRY(cudaCheck(cudaMemsetAsync(N->loss.p, 0, sizeof(double), N->stream), "memset"));
+	PWA_TRY(mlpBackward(N, (int)B, N->loss.as<double>()));
 	if (loss)
 		PWA_TRY(cudaCheck(cudaMemcpyAsync(loss, N->loss.p, sizeof(double), cudaMemcpyDeviceToHost, N->stream),
 		                  "download"));
@@ -351,7 +377,7 @@ int pwa_mlp_train(pwa_mlp* N, const float* X, const float* T, uint64_t nSamples,
 	PWA_TRY(mlpEnsureBatch(N, B));
 	cudaStream_t s = N->stream;
 	// training set on the device: inputs as BF16, targets FP32
-	PWA_TRY(N->trainX.alloc(nSamples * N->nIn * 2, "MLP training inputs"));
+	PWA_TRY(N->trainX.alloc(nSamples * N->nInP * 2, "MLP training inputs"));
 	PWA_TRY(N->trainT.alloc(nSamples * N->nOut * 4, "MLP training targets"));
 	{
 		const uint64_t chunk = std::max<uint64_t>(1, (64ull << 20) / ((uint64_t)N->nIn * 4));
@@ -361,7 +387,7 @@ int pwa_mlp_train(pwa_mlp* N, const float* X, const float* T, uint64_t nSamples,
 			const uint64_t n = std::min(chunk, nSamples - r);
 			PWA_TRY(cudaCheck(cudaMemcpyAsync(x32.p, X + r * N->nIn, n * N->nIn * 4, cudaMemcpyHostToDevice, s),
 			                  "upload"));
-			PWA_TRY(launchToBf16(x32.as<float>(), N->trainX.as<uint16_t>() + r * N->nIn, n * N->nIn, s));
+			PWA_TRY(launchToBf16(x32.as<float>(), N->trainX.as<uint16_t>() + r * N->nInP, n, N->nIn, N->nInP, s));
 			PWA_TRY(cudaCheck(cudaStreamSynchronize(s), "upload"));
 		}
 	}
@@ -373,22 +399,30 @@ int pwa_mlp_train(pwa_mlp* N, const float* X, const float* T, uint64_t nSamples,
 	DevBuf dPerm;
 	PWA_TRY(dPerm.alloc(nSamples * 4, "MLP permutation"));
 	const uint64_t steps = nSamples / (uint64_t)B;
+	// every step's error on the device, read once per epoch and added up in
+	// step order (reading each took a synchronisation per step)
+	DevBuf dLoss;
+	PWA_TRY(dLoss.alloc(std::max<uint64_t>(1, steps) * sizeof(double), "MLP step errors"));
+	std::vector<double> stepLoss(steps);
 	for (uint32_t ep = 0; ep < epochs; ++ep) {
 		std::shuffle(perm.begin(), perm.end(), rng);
 		PWA_TRY(cudaCheck(cudaMemcpyAsync(dPerm.p, perm.data(), nSamples * 4, cudaMemcpyHostToDevice, s), "upload"));
-		double epochLoss = 0.;
+		PWA_TRY(cudaCheck(cudaMemsetAsync(dLoss.p, 0, dLoss.bytes, s), "memset"));
 		for (uint64_t st = 0; st < steps; ++st) {
 			const uint32_t* idx = dPerm.as<uint32_t>() + st * B;
-			PWA_TRY(launchGatherRows(N->trainX.p, idx, B, (size_t)N->nIn * 2, N->x16.p, s));
+			PWA_TRY(launchGatherRows(N->trainX.p, idx, B, (size_t)N->nInP * 2, N->x16.p, s));
 			PWA_TRY(launchGatherRows(N->trainT.p, idx, B, (size_t)N->nOut * 4, N->t32.p, s));
 			PWA_TRY(mlpForward(N, B));
-			PWA_TRY(mlpBackward(N, B));
-			double l = 0.;
-			PWA_TRY(cudaCheck(cudaMemcpyAsync(&l, N->loss.p, sizeof(double), cudaMemcpyDeviceToHost, s), "download"));
-			PWA_TRY(cudaCheck(cudaStreamSynchronize(s), "MLP step"));
-			epochLoss += l;
+			PWA_TRY(mlpBackward(N, B, dLoss.as<double>() + st));
 			PWA_TRY(mlpAdam(N, lr));
 		}
+		if (steps)
+			PWA_TRY(cudaCheck(cudaMemcpyAsync(stepLoss.data(), dLoss.p, steps * sizeof(double), cudaMemcpyDeviceToHost, s),
+			                  "download"));
+		PWA_TRY(cudaCheck(cudaStreamSynchronize(s), "MLP epoch"));
+		double epochLoss = 0.;
+		for (double l : stepLoss)
+			epochLoss += l;
 		if (lossHistory)
 			lossHistory[ep] = epochLoss / (double)std::max<uint64_t>(1, steps);
 		PWA_TRY(mlpCheckDevice(N));

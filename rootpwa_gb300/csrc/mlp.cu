@@ -5,17 +5,28 @@
 //
 // One tensor-core GEMM kernel serves every product: C[M][N] = sum_k A(m, k)
 // B(k, n) with A and B read through strides (so that X W^T, dY W and dY^T X
-// are the same kernel).  128 x 128 output tiles; per K step of 64 the four
-// loader warps read both operand tiles from global memory (along whichever
-// dimension is contiguous) and write them in the canonical K-major
-// 128-byte-swizzled layout, one thread issues four tcgen05.mma kind::f16
-// (BF16 operands, M = N = 128, K = 16) into an FP32 accumulator in tensor
-// memory (128 columns), two operand stages alternate.  The product is split
-// into K slices, one block per (tile, slice), so that the grid covers the
-// GPU (the batch has 256 rows, the layers 102 to 512 columns); the loader
+// are the same kernel).  Every BF16 matrix is stored with its rows padded
+// with zeros to a multiple of eight elements, so that all operand loads are
+// 16-byte vectors (the 5203-wide input rows would otherwise start at odd
+// two-byte offsets).  128 x 128 output tiles; per K step of 64 the
+// four loader warps read both operand tiles and write them in the canonical
+// K-major 128-byte-swizzled layout (8 x 8 blocks transposed in registers where
+// the other dimension is contiguous), one thread issues four tcgen05.mma
+// kind::f16 (BF16 operands, M = N = 128, K = 16) into an FP32 accumulator in
+// tensor memory (128 columns), two operand stages alternate.  The product is
+// split into K slices, one block per (tile, slice), so that the grid covers
+// the GPU (the batch has 256 rows, the layers 102 to 512 columns); the loader
 // warps then move the accumulator to the slice's FP32 partials, and a second
 // kernel sums the slices in slice order (deterministic) and applies the
 // epilogue: bias, relu or a relu mask, FP32 and/or BF16 stores.
+//
+// What bounds it: latency (a block has one to three K steps) and, for the two
+// products over the 5203 inputs, the slices' partials in L2.  256 rows of
+// 5203-512-512-102, caches cold: the products took 22 us on average with
+// single-element operand loads and one row per lane in the drain; vector
+// loads alone left 12 to 15 us and, for the first layer and its weight
+// gradient, 32 and 44; with rows stored whole, 7 and 13 and 16.  A training
+// step takes 178 us against 352 before (Adam's 83 MB among them: 24 us).
 
 #include "pwa_internal.h"
 #include "tcgen05.cuh"
@@ -40,59 +51,67 @@ constexpr size_t kTcSmem = 1024 + 2u * kTcStages * kTcOpBytes + 128;
 // bias, relu, relu mask and the FP32 / BF16 stores of one output element
 __device__ __forceinline__ void mlpEpilogue(const MlpGemm& g, int m, int n, float v)
 {
-	const size_t o = (size_t)m * g.N + n;
+	const size_t o = (size_t)m * g.N + n, o16 = (size_t)m * g.ld16 + n;
 	if (g.bias)
 		v += g.bias[n];
 	if (g.relu)
 		v = fmaxf(v, 0.f);
 	const __nv_bfloat16* mask = reinterpret_cast<const __nv_bfloat16*>(g.mask);
-	if (mask && !(__bfloat162float(mask[o]) > 0.f))
+	if (mask && !(__bfloat162float(mask[o16]) > 0.f))
 		v = 0.f;
 	if (g.C32)
 		g.C32[o] = v;
 	if (g.C16)
-		reinterpret_cast<__nv_bfloat16*>(g.C16)[o] = __float2bfloat16_rn(v);
+		reinterpret_cast<__nv_bfloat16*>(g.C16)[o16] = __float2bfloat16_rn(v);
 }
 
 // one 128 x 64 operand tile in the K-major swizzled layout: row r, k of
-// element (r, k) = X[r * ldr + k * ldk] of rows r0.., k0.. (zero beyond
-// nR rows or kEnd); 128 loader threads, each storing 16-byte chunks of 8 k
+// element (r, k) = X[r * ldr + k * ldk] of rows r0.., k0.. (zero beyond nR
+// rows or kEnd); one of ldr, ldk is 1, the other a multiple of 8, and X is
+// 16-byte aligned with zeros after the last element of a padded row.  128
+// loader threads, eight 16-byte loads each.
 __device__ __forceinline__ void loadTile(unsigned char* dst, const uint16_t* X, size_t ldr, size_t ldk, int contigK,
                                          int r0, int nR, int k0, int kEnd, int t)
 {
+	const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 	if (contigK) {
-		// thread t: chunks t, t + 128, ... (8 per thread): row c / 8, k-chunk c % 8
-#pragma unroll 2
+		// thread t: chunks t, t + 128, ...: row c / 8, k-chunk c % 8.  kEnd is a
+		// multiple of 8 or the end of the padded rows
+		uint4 v[8];
+#pragma unroll
 		for (int j = 0; j < 8; ++j) {
 			const int c = t + 128 * j, r = c >> 3, kc = (c & 7) * 8;
-			uint32_t w[4] = {0u, 0u, 0u, 0u};
-			if (r0 + r < nR) {
-				const uint16_t* src = X + (size_t)(r0 + r) * ldr;
+			v[j] = (r0 + r < nR && k0 + kc < kEnd)
+			           ? __ldg(reinterpret_cast<const uint4*>(X + (size_t)(r0 + r) * ldr + k0 + kc))
+			           : zero;
+		}
 #pragma unroll
-				for (int i = 0; i < 8; ++i) {
-					const int k = k0 + kc + i;
-					const uint32_t v = k < kEnd ? src[k] : 0u;
-					w[i >> 1] |= v << (16 * (i & 1));
-				}
-			}
-			*reinterpret_cast<uint4*>(dst + swzOffset16(r, kc)) = make_uint4(w[0], w[1], w[2], w[3]);
+		for (int j = 0; j < 8; ++j) {
+			const int c = t + 128 * j, r = c >> 3, kc = (c & 7) * 8;
+			*reinterpret_cast<uint4*>(dst + swzOffset16(r, kc)) = v[j];
 		}
 	} else {
-		// thread t: row t, all 8 k-chunks (neighbouring threads read neighbouring rows)
-		const int r = t;
-		const bool in = r0 + r < nR;
-#pragma unroll 2
-		for (int kc = 0; kc < kTcK; kc += 8) {
-			uint32_t w[4] = {0u, 0u, 0u, 0u};
-			if (in) {
+		// thread t: the 8 x 8 block of rows 8 (t / 8) .. and k 8 (t % 8) ..:
+		// one load per k, then each row's eight k together
+		const int rb = (t >> 3) * 8, kb = (t & 7) * 8;
+		uint32_t v[8][4];
 #pragma unroll
-				for (int i = 0; i < 8; ++i) {
-					const int k = k0 + kc + i;
-					const uint32_t v = k < kEnd ? X[(size_t)(r0 + r) * ldr + (size_t)k * ldk] : 0u;
-					w[i >> 1] |= v << (16 * (i & 1));
-				}
-			}
-			*reinterpret_cast<uint4*>(dst + swzOffset16(r, kc)) = make_uint4(w[0], w[1], w[2], w[3]);
+		for (int i = 0; i < 8; ++i) {
+			const uint4 q = (r0 + rb < nR && k0 + kb + i < kEnd)
+			                    ? __ldg(reinterpret_cast<const uint4*>(X + (size_t)(k0 + kb + i) * ldk + r0 + rb))
+			                    : zero;
+			v[i][0] = q.x;
+			v[i][1] = q.y;
+			v[i][2] = q.z;
+			v[i][3] = q.w;
+		}
+#pragma unroll
+		for (int r = 0; r < 8; ++r) {
+			uint32_t w[4];
+#pragma unroll
+			for (int i = 0; i < 4; ++i)
+				w[i] = __byte_perm(v[2 * i][r >> 1], v[2 * i + 1][r >> 1], (r & 1) ? 0x7632 : 0x5410);
+			*reinterpret_cast<uint4*>(dst + swzOffset16(rb + r, kb)) = make_uint4(w[0], w[1], w[2], w[3]);
 		}
 	}
 }
@@ -165,8 +184,12 @@ __global__ void __launch_bounds__(kTcThreads) mlpGemmTcKernel(const MlpGemm g, i
 		}
 		if (ok) {
 			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-			const int m = m0 + warp * 32 + lane;
-			float* out = g.work + ((size_t)blockIdx.z * g.M + (size_t)(m < g.M ? m : 0)) * g.N;
+			// through shared memory (the operand stages are done with), so that
+			// a row's 128 columns are stored together: one lane per row would
+			// write every 32-byte sector eight times.  16-byte piece q of row r
+			// at q ^ r: conflict-free both ways.
+			float4* const rows = reinterpret_cast<float4*>(opA) + warp * 32 * 32;
+#pragma unroll 2
 			for (int c = 0; c < kTcTile; c += 16) {
 				uint32_t r[16];
 				if (nSteps > 0) {
@@ -177,12 +200,20 @@ __global__ void __launch_bounds__(kTcThreads) mlpGemmTcKernel(const MlpGemm g, i
 					for (int i = 0; i < 16; ++i)
 						r[i] = 0u;
 				}
-				if (m < g.M)
 #pragma unroll
-					for (int i = 0; i < 16; ++i)
-						if (n0 + c + i < g.N)
-							out[n0 + c + i] = __uint_as_float(r[i]);
+				for (int i = 0; i < 4; ++i)
+					rows[lane * 32 + ((c / 4 + i) ^ lane)] =
+					    make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]),
+					                __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
 			}
+			__syncwarp();
+			const int ldw = mlpWorkLd(g.N), n = n0 + 4 * lane, mw = m0 + warp * 32;
+			float* out = g.work + ((size_t)blockIdx.z * g.M + mw) * ldw + n;
+			if (n < ldw)
+#pragma unroll 8
+				for (int r = 0; r < 32; ++r)
+					if (mw + r < g.M)
+						*reinterpret_cast<float4*>(out + (size_t)r * ldw) = rows[r * 32 + (lane ^ r)];
 		}
 	} else if (lane == 0) {
 		// ---- MMA issuer ----
@@ -215,33 +246,65 @@ __global__ void __launch_bounds__(kTcThreads) mlpGemmTcKernel(const MlpGemm g, i
 	}
 }
 
-// sum of the K slices' partials in slice order, then the epilogue
-__global__ void mlpSplitReduceKernel(const MlpGemm g)
+// sum of the K slices' partials in slice order, then the epilogue: four
+// columns per thread
+__global__ void __launch_bounds__(128) mlpSplitReduceKernel(const MlpGemm g)
 {
-	const size_t total = (size_t)g.M * g.N;
-	for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < total; o += (size_t)gridDim.x * blockDim.x) {
-		float v = 0.f;
-		for (int z = 0; z < g.splitK; ++z)
-			v += g.work[(size_t)z * total + o];
-		mlpEpilogue(g, (int)(o / g.N), (int)(o % g.N), v);
+	const int ldw = mlpWorkLd(g.N), n = 4 * (blockIdx.x * 128 + threadIdx.x);
+	if (n >= g.N)
+		return;
+	const size_t slice = (size_t)g.M * ldw;
+	for (int m = blockIdx.y; m < g.M; m += gridDim.y) {
+		const float4* p = reinterpret_cast<const float4*>(g.work + (size_t)m * ldw + n);
+		float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+		for (int z = 0; z < g.splitK; ++z) {
+			const float4 q = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + z * slice));
+			v[0] += q.x;
+			v[1] += q.y;
+			v[2] += q.z;
+			v[3] += q.w;
+		}
+#pragma unroll
+		for (int i = 0; i < 4; ++i)
+			if (n + i < g.N)
+				mlpEpilogue(g, m, n + i, v[i]);
 	}
 }
 
-// column sums of an FP32 [M][N] matrix (bias gradients)
-__global__ void colSumKernel(const float* X, int M, int N, float* out)
+// column sums of an FP32 [M][N] matrix (bias gradients), rows in order: the
+// block brings 256 rows of 32 columns to shared memory at a time, one warp adds
+// them (with that warp's own loads, 64 rows in flight, 256 rows took 8 us).
+constexpr int kColRows = 256;
+__global__ void __launch_bounds__(256) colSumKernel(const float* __restrict__ X, int M, int N, float* out)
 {
-	const int n = blockIdx.x * blockDim.x + threadIdx.x;
-	if (n >= N)
-		return;
+	__shared__ float tile[kColRows][32];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = blockIdx.x * 32 + lane;
 	float s = 0.f;
-	for (int m = 0; m < M; ++m)
-		s += X[(size_t)m * N + n];
-	out[n] = s;
+	for (int m0 = 0; m0 < M; m0 += kColRows) {
+		const int rows = min(kColRows, M - m0);
+		float v[kColRows / 8];
+#pragma unroll
+		for (int i = 0; i < kColRows / 8; ++i)
+			v[i] = n < N && warp + 8 * i < rows ? __ldg(X + (size_t)(m0 + warp + 8 * i) * N + n) : 0.f;
+#pragma unroll
+		for (int i = 0; i < kColRows / 8; ++i)
+			tile[warp + 8 * i][lane] = v[i];
+		__syncthreads();
+		if (warp == 0) {
+#pragma unroll 32
+			for (int i = 0; i < rows; ++i)
+				s += tile[i][lane];
+		}
+		__syncthreads();
+	}
+	if (warp == 0 && n < N)
+		out[n] = s;
 }
 
 // squared error sum over n values (FP64 total, times `scale`) and
-// dY = 2 (Y - T) scale
-__global__ void mseKernel(const float* Y, const float* T, int n, float scale, float* dY32, uint16_t* dY16,
+// dY = 2 (Y - T) scale (BF16 copy in rows of ld16)
+__global__ void mseKernel(const float* Y, const float* T, int n, int N, int ld16, float scale, float* dY32, uint16_t* dY16,
                           double* loss)
 {
 	double part = 0.;
@@ -251,7 +314,7 @@ __global__ void mseKernel(const float* Y, const float* T, int n, float scale, fl
 		part += (double)d * d;
 		const float gval = 2.f * d * scale;
 		dY32[i] = gval;
-		d16[i] = __float2bfloat16_rn(gval);
+		d16[(size_t)(i / N) * ld16 + i % N] = __float2bfloat16_rn(gval);
 	}
 	for (int o = 16; o > 0; o >>= 1)
 		part += __shfl_xor_sync(0xffffffffu, part, o);
@@ -259,39 +322,97 @@ __global__ void mseKernel(const float* Y, const float* T, int n, float scale, fl
 		atomicAdd(loss, part * (double)scale);
 }
 
-// Adam on FP32 master weights; refreshes the BF16 copy
-__global__ void adamKernel(float* w, const float* g, float* m, float* v, uint16_t* w16, size_t n, float lr, float b1,
-                           float b2, float eps, float c1, float c2)
+// element i of the parameter vector in the padded BF16 weights, or -1 (bias)
+__device__ __forceinline__ long long w16Index(const MlpWeights& w, size_t i)
+{
+#pragma unroll
+	for (int l = 0; l < 3; ++l)
+		if (i >= w.from[l] && i < w.from[l] + (size_t)w.rows[l] * w.cols[l]) {
+			const size_t q = i - w.from[l];
+			const size_t r = q <= 0xffffffffull ? (size_t)((uint32_t)q / (uint32_t)w.cols[l]) : q / w.cols[l];
+			return (long long)(w.to[l] + r * w.ld[l] + (q - r * w.cols[l]));
+		}
+	return -1;
+}
+
+// Adam on FP32 master weights; refreshes the BF16 copy.  Four parameters per
+// thread (the arrays come from the allocator, 16-byte aligned).  The moments'
+// fused multiply-adds are written out: a run's weights do not depend on which
+// product the compiler fuses.
+__global__ void __launch_bounds__(256) adamKernel(float* w, const float* __restrict__ g, float* m, float* v,
+                                                  uint16_t* w16, size_t n, float lr, float b1, float b2, float eps,
+                                                  float c1, float c2, const MlpWeights map)
 {
 	__nv_bfloat16* o16 = reinterpret_cast<__nv_bfloat16*>(w16);
-	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-		const float gi = g[i];
-		const float mi = b1 * m[i] + (1.f - b1) * gi;
-		const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-		m[i] = mi;
-		v[i] = vi;
-		const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-		w[i] = wi;
-		o16[i] = __float2bfloat16_rn(wi);
+	const size_t i0 = 4 * (blockIdx.x * (size_t)256 + threadIdx.x);
+	if (i0 >= n)
+		return;
+	const int k = (int)min((size_t)4, n - i0);
+	float gi[4], mi[4], vi[4], wi[4];
+	if (k == 4) {
+		*reinterpret_cast<float4*>(gi) = *reinterpret_cast<const float4*>(g + i0);
+		*reinterpret_cast<float4*>(mi) = *reinterpret_cast<const float4*>(m + i0);
+		*reinterpret_cast<float4*>(vi) = *reinterpret_cast<const float4*>(v + i0);
+		*reinterpret_cast<float4*>(wi) = *reinterpret_cast<const float4*>(w + i0);
+	} else {
+		for (int j = 0; j < k; ++j) {
+			gi[j] = g[i0 + j];
+			mi[j] = m[i0 + j];
+			vi[j] = v[i0 + j];
+			wi[j] = w[i0 + j];
+		}
+	}
+#pragma unroll
+	for (int j = 0; j < 4; ++j) {
+		mi[j] = __fmaf_rn(1.f - b1, gi[j], __fmul_rn(b1, mi[j]));
+		vi[j] = __fmaf_rn(__fmul_rn(1.f - b2, gi[j]), gi[j], __fmul_rn(b2, vi[j]));
+		wi[j] = wi[j] - lr * (mi[j] / c1) / (sqrtf(vi[j] / c2) + eps);
+	}
+	if (k == 4) {
+		*reinterpret_cast<float4*>(m + i0) = *reinterpret_cast<float4*>(mi);
+		*reinterpret_cast<float4*>(v + i0) = *reinterpret_cast<float4*>(vi);
+		*reinterpret_cast<float4*>(w + i0) = *reinterpret_cast<float4*>(wi);
+	} else {
+		for (int j = 0; j < k; ++j) {
+			m[i0 + j] = mi[j];
+			v[i0 + j] = vi[j];
+			w[i0 + j] = wi[j];
+		}
+	}
+	for (int j = 0; j < k; ++j) {
+		const long long o = w16Index(map, i0 + j);
+		if (o >= 0)
+			o16[o] = __float2bfloat16_rn(wi[j]);
 	}
 }
 
-__global__ void toBf16Kernel(const float* x, uint16_t* y, size_t n)
+__global__ void weights16Kernel(const float* w, uint16_t* w16, size_t n, const MlpWeights map)
 {
-	__nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(y);
-	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-		o[i] = __float2bfloat16_rn(x[i]);
+	__nv_bfloat16* o16 = reinterpret_cast<__nv_bfloat16*>(w16);
+	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+		const long long o = w16Index(map, i);
+		if (o >= 0)
+			o16[o] = __float2bfloat16_rn(w[i]);
+	}
 }
 
-// rows idx[r] of src [*][rowLen] -> dst [r][rowLen] (element size esz bytes)
-__global__ void gatherRowsKernel(const unsigned char* src, const uint32_t* idx, int rows, size_t rowBytes,
-                                 unsigned char* dst)
+// rows of `cols` FP32 values into BF16 rows of ld >= cols (zeros after them)
+__global__ void toBf16Kernel(const float* x, uint16_t* y, size_t rows, int cols, int ld)
+{
+	__nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(y);
+	for (size_t r = blockIdx.y; r < rows; r += gridDim.y)
+		for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ld; c += gridDim.x * blockDim.x)
+			o[r * ld + c] = __float2bfloat16_rn(c < cols ? x[r * cols + c] : 0.f);
+}
+
+// rows idx[r] of src -> dst [r] in units of U (16 or 4 bytes)
+template <typename U>
+__global__ void gatherRowsKernel(const U* __restrict__ src, const uint32_t* idx, int rows, int units, U* dst)
 {
 	for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-		const unsigned char* s = src + (size_t)idx[r] * rowBytes;
-		unsigned char* d = dst + (size_t)r * rowBytes;
-		for (size_t i = threadIdx.x; i < rowBytes; i += blockDim.x)
-			d[i] = s[i];
+		const U* s = src + (size_t)idx[r] * units;
+		for (int i = threadIdx.x; i < units; i += blockDim.x)
+			dst[(size_t)r * units + i] = s[i];
 	}
 }
 
@@ -327,51 +448,63 @@ int launchMlpGemm(const MlpGemm& g, cudaStream_t s)
 	PWA_CHECK(cudaCheck(cudaGetLastError(), "MLP GEMM launch"));
 	MlpGemm r = g;
 	r.splitK = slices;
-	const size_t total = (size_t)g.M * g.N;
-	const int blocks = (int)std::min<size_t>(4096, (total + 255) / 256);
-	mlpSplitReduceKernel<<<blocks, 256, 0, s>>>(r);
+	const dim3 rgrid((g.N + 511) / 512, std::min(g.M, 65535));
+	mlpSplitReduceKernel<<<rgrid, 128, 0, s>>>(r);
 	countLaunches(1);
 	return cudaCheck(cudaGetLastError(), "MLP split-K reduce launch");
 }
 
 int launchColSum(const float* X, int M, int N, float* out, cudaStream_t s)
 {
-	colSumKernel<<<(N + 127) / 128, 128, 0, s>>>(X, M, N, out);
+	colSumKernel<<<(N + 31) / 32, 256, 0, s>>>(X, M, N, out);
 	countLaunches(1);
 	return cudaCheck(cudaGetLastError(), "column sum launch");
 }
 
-int launchMse(const float* Y, const float* T, int n, float scale, float* dY32, uint16_t* dY16, double* loss,
-              cudaStream_t s)
+int launchMse(const float* Y, const float* T, int n, int N, int ld16, float scale, float* dY32, uint16_t* dY16,
+              double* loss, cudaStream_t s)
 {
 	const int blocks = std::min(1024, std::max(1, (n + 255) / 256));
-	mseKernel<<<blocks, 256, 0, s>>>(Y, T, n, scale, dY32, dY16, loss);
+	mseKernel<<<blocks, 256, 0, s>>>(Y, T, n, N, ld16, scale, dY32, dY16, loss);
 	countLaunches(1);
 	return cudaCheck(cudaGetLastError(), "MSE launch");
 }
 
 int launchAdam(float* w, const float* g, float* m, float* v, uint16_t* w16, size_t n, float lr, float b1, float b2,
-               float eps, float c1, float c2, cudaStream_t s)
+               float eps, float c1, float c2, const MlpWeights& map, cudaStream_t s)
 {
-	const int blocks = (int)std::min<size_t>(2048, std::max<size_t>(1, (n + 255) / 256));
-	adamKernel<<<blocks, 256, 0, s>>>(w, g, m, v, w16, n, lr, b1, b2, eps, c1, c2);
+	const unsigned blocks = (unsigned)std::max<size_t>(1, (n + 1023) / 1024);
+	adamKernel<<<blocks, 256, 0, s>>>(w, g, m, v, w16, n, lr, b1, b2, eps, c1, c2, map);
 	countLaunches(1);
 	return cudaCheck(cudaGetLastError(), "Adam launch");
 }
 
-int launchToBf16(const float* x, uint16_t* y, size_t n, cudaStream_t s)
+int launchWeights16(const float* w, uint16_t* w16, size_t n, const MlpWeights& map, cudaStream_t s)
 {
 	const int blocks = (int)std::min<size_t>(4096, std::max<size_t>(1, (n + 255) / 256));
-	toBf16Kernel<<<blocks, 256, 0, s>>>(x, y, n);
+	weights16Kernel<<<blocks, 256, 0, s>>>(w, w16, n, map);
+	countLaunches(1);
+	return cudaCheck(cudaGetLastError(), "bf16 weights launch");
+}
+
+int launchToBf16(const float* x, uint16_t* y, size_t rows, int cols, int ld, cudaStream_t s)
+{
+	const dim3 grid((unsigned)((ld + 255) / 256), (unsigned)std::min<size_t>(rows, 4096));
+	toBf16Kernel<<<grid, 256, 0, s>>>(x, y, rows, cols, ld);
 	countLaunches(1);
 	return cudaCheck(cudaGetLastError(), "bf16 conversion launch");
 }
 
 int launchGatherRows(const void* src, const uint32_t* idx, int rows, size_t rowBytes, void* dst, cudaStream_t s)
 {
+	// rows of whole 16-byte units, or of FP32 values
 	const int blocks = std::min(4096, std::max(1, rows));
-	gatherRowsKernel<<<blocks, 256, 0, s>>>(static_cast<const unsigned char*>(src), idx, rows, rowBytes,
-	                                        static_cast<unsigned char*>(dst));
+	if (rowBytes % 16 == 0)
+		gatherRowsKernel<<<blocks, 256, 0, s>>>(static_cast<const uint4*>(src), idx, rows, (int)(rowBytes / 16),
+		                                        static_cast<uint4*>(dst));
+	else
+		gatherRowsKernel<<<blocks, 256, 0, s>>>(static_cast<const uint32_t*>(src), idx, rows, (int)(rowBytes / 4),
+		                                        static_cast<uint32_t*>(dst));
 	countLaunches(1);
 	return cudaCheck(cudaGetLastError(), "row gather launch");
 }

@@ -298,8 +298,20 @@ int launchCountActive(const int* status, int Q, int* active, unsigned* nActive, 
 // ---------------------------------------------------------------------------
 // Warm-start network kernels (mlp.cu)
 // ---------------------------------------------------------------------------
+// BF16 matrices are stored in rows padded with zeros to a multiple of 8
+// elements (16 bytes): padded row length of n elements
+inline int mlpPad(int n) { return (n + 7) / 8 * 8; }
+// row length of the K slices' FP32 partials
+__host__ __device__ inline int mlpWorkLd(int n) { return (n + 3) / 4 * 4; }
+// the three weight matrices in the parameter vector (from: offset, rows x
+// cols) and in the padded BF16 copy (to: offset, ld)
+struct MlpWeights {
+	size_t from[3], to[3];
+	int rows[3], cols[3], ld[3];
+};
 // C[M][N] = sum_k A(m, k) B(k, n) (+ bias[n], relu, relu mask), BF16 operands
-// A(m, k) = A[m * lda_m + k * lda_k], B(k, n) = B[k * ldb_k + n * ldb_n]
+// A(m, k) = A[m * lda_m + k * lda_k], B(k, n) = B[k * ldb_k + n * ldb_n]; of
+// either pair of strides one is 1 and the other a multiple of 8
 struct MlpGemm {
 	int M, N, K;
 	const uint16_t* A;
@@ -310,22 +322,25 @@ struct MlpGemm {
 	int bContigK;        // 1 when ldb_k == 1
 	const float* bias;   // [N] or null
 	int relu;
-	const uint16_t* mask;  // BF16 [M][N]: zero the output where mask <= 0, or null
+	const uint16_t* mask;  // BF16 [M][ld16]: zero the output where mask <= 0, or null
 	float* C32;          // FP32 [M][N] or null
-	uint16_t* C16;       // BF16 [M][N] or null
+	uint16_t* C16;       // BF16 [M][ld16] or null
+	int ld16;
 	int splitK;          // K slices (whole K steps of 64): FP32 partials in work, then the epilogue kernel
-	float* work;         // FP32 [splitK][M][N]
+	float* work;         // FP32 [splitK][M][mlpWorkLd(N)]
 	unsigned* devErr;    // device error flag (a bounded wait of the tensor-core kernel expired)
 };
 // K slices for the tensor-core GEMM (its blocks cover the SMs about twice)
 int mlpGemmSplit(const MlpGemm& g, int numSMs);
 int launchMlpGemm(const MlpGemm& g, cudaStream_t s);
 int launchColSum(const float* X, int M, int N, float* out, cudaStream_t s);
-int launchMse(const float* Y, const float* T, int n, float scale, float* dY32, uint16_t* dY16, double* loss,
-              cudaStream_t s);
+int launchMse(const float* Y, const float* T, int n, int N, int ld16, float scale, float* dY32, uint16_t* dY16,
+              double* loss, cudaStream_t s);
 int launchAdam(float* w, const float* g, float* m, float* v, uint16_t* w16, size_t n, float lr, float b1, float b2,
-               float eps, float c1, float c2, cudaStream_t s);
-int launchToBf16(const float* x, uint16_t* y, size_t n, cudaStream_t s);
+               float eps, float c1, float c2, const MlpWeights& map, cudaStream_t s);
+int launchWeights16(const float* w, uint16_t* w16, size_t n, const MlpWeights& map, cudaStream_t s);
+// rows of cols FP32 values -> BF16 rows of ld elements, zeros after the values
+int launchToBf16(const float* x, uint16_t* y, size_t rows, int cols, int ld, cudaStream_t s);
 int launchGatherRows(const void* src, const uint32_t* idx, int rows, size_t rowBytes, void* dst, cudaStream_t s);
 
 // ---------------------------------------------------------------------------
