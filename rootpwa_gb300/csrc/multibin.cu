@@ -10,15 +10,15 @@
 // evaluate each problem with its bin's own FdF kernel (fdf_kernels.cu,
 // returning at once for converged problems) and gatherEvalKernel.  Packed
 // layouts:
-//   fdfBatchKernel   -- persistent blocks walk a list of work items
-//                       (bin, group of SG starts, range of 128-event tiles);
+//   fdfBatch32Kernel -- persistent blocks walk a list of work items
+//                       (bin, group of 32 starts, range of 128-event tiles);
 //                       each tile is loaded once by a bulk copy and used for all
-//                       SG starts: phase 1 forms S_{s,e} = sum_w V_{s,w} A_{w,e},
+//                       starts: phase 1 forms S_{s,e} = sum_w V_{s,w} A_{w,e},
 //                       L = |S|^2 + V_flat^2, -ln L and c S (c = -2/L); phase 2
 //                       G_{s,w} += sum_e c S_{s,e} conj(A_{w,e});
 //                       per-thread FP32 (compensated for -ln L and c) over up
-//                       to 8 tiles, then FP64; FP64 partials per item.
-//                       Groups of 32 starts: two tile stages, one block per SM;
+//                       to 8 tiles, then FP64; FP64 partials per item.  Two
+//                       tile stages, one block per SM;
 //   fdfBatch8Kernel  -- the same for groups of 8 starts (little work per
 //                       tile): register-blocked phases over a quarter of the
 //                       waves or events per thread, combined by shuffles; one
@@ -38,6 +38,7 @@
 #include "device_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace pwa {
 namespace {
@@ -46,59 +47,76 @@ constexpr int kBThreads = 256;
 constexpr int kBE = 128;     // events per tile (the amplitude store's block)
 constexpr int kBFold = 8;    // tiles summed in FP32 before the FP64 fold
 
+// ---- start groups of 32 ----
+// 512 threads (16 warps, 128 registers), one block per SM, two tile stages.
+// Phase 1: a thread forms the sums of 2 starts x 4 events over the waves;
+// phase 2: of 2 starts x 2 waves over the events.  Lane bits 0, 2, 3 ("quad")
+// select the starts, bits 1 and 4 ("four") the events or the waves: every
+// 16-byte load then has its address in common with lane ^ 1 or lane ^ 2 and
+// takes two passes of the shared-memory pipe (with the starts in bits 0..2 the
+// V and c S loads take four).  A thread's waves are 32 apart, so that the
+// waves beyond 32 are spread over all four schedulers' warps.
+//
+// What bounds it: the FP32 pipe (packed multiply-adds, two cycles each) and the
+// shared-memory pipe about equally, with one barrier per tile.  A tile of 50
+// waves takes 23 k cycles of an SM (14.6 k if only the multiply-adds counted);
+// eight warps of 255 registers (4 starts x 4 events, 4 starts x 2 waves) took
+// 28 k: their two warps per scheduler did not hide the latencies.  Eight warps
+// per phase working on successive tiles took 27 k (the c S hand-over between
+// them is exposed; a third tile stage or a second c S buffer does not fit).
+// 24 bins x 64 starts x 50 waves (1.3 M events): a call took 2.19 ms, now 1.89
+// (this kernel 1.65).
+constexpr int kB32Threads = 512;
+constexpr int kB32Group = 32;
+
 struct BatchSmem {
 	size_t stages, vs, ts, flat, bars, total;
 };
 
-__host__ __device__ inline BatchSmem batchSmem(int W, int SG, int NST)
+__host__ __device__ inline BatchSmem batchSmem(int W)
 {
 	BatchSmem L{};
 	auto up = [](size_t x) { return (x + 127) & ~size_t(127); };
 	L.stages = 0;
-	L.vs = up((size_t)NST * W * kBE * 8);
-	L.ts = up(L.vs + (size_t)W * SG * 16);
-	L.flat = up(L.ts + (size_t)2 * kBE * SG * 8);
-	L.bars = up(L.flat + (size_t)SG * 4);
+	L.vs = up((size_t)2 * W * kBE * 8);
+	L.ts = up(L.vs + (size_t)W * kB32Group * 8);
+	L.flat = up(L.ts + (size_t)2 * kBE * kB32Group * 8);
+	L.bars = up(L.flat + (size_t)kB32Group * 4);
 	L.total = L.bars + 2 * 8 + 128;
 	return L;
 }
 
-// SG starts per group; phase 1: SPT starts x EPT events per thread;
-// phase 2: SPT2 starts x WPT waves per thread (waves < 64).  NST tile stages
-// per block: 2 (the next tile loads while this one is used) or 1 (MINB
-// blocks per SM take turns instead).  Instantiated for groups of 32 starts
-// (two stages, one block per SM); groups of 8 use fdfBatch8Kernel below.
-template <int SG, int SPT, int EPT, int SPT2, int WPT, int NST, int MINB>
-__global__ void __launch_bounds__(kBThreads, MINB) fdfBatchKernel(const BatchArgs a)
+__global__ void __launch_bounds__(kB32Threads, 1) fdfBatch32Kernel(const BatchArgs a)
 {
-	static_assert(NST == 1 || NST == 2, "one or two tile stages");
-	static_assert((SG / SPT) * (kBE / EPT) == kBThreads, "phase-1 mapping");
-	static_assert((SG / SPT2) * (64 / WPT) == kBThreads, "phase-2 mapping");
-	static_assert(EPT % 2 == 0 && SPT2 % 2 == 0 && SPT % 2 == 0, "paired loads");
-	static_assert(SPT == SPT2, "both phases group the starts in the same quads");
-	constexpr int NQ = SG / SPT;  // start groups of SPT (phase-1 sq, phase-2 sp)
+	constexpr int SG = kB32Group;
+	static_assert(kBE == 128, "event groups of 4, rows rotated by 4 (w mod 4) events");
 	extern __shared__ __align__(128) unsigned char smem[];
 	const int W = a.W, P = a.P;
-	const BatchSmem lay = batchSmem(W, SG, NST);
-	float2* stages = reinterpret_cast<float2*>(smem + lay.stages);  // [NST][W][kBE]
-	// V of start s = q * SPT + i at [w][i][q] (vx, vx, vy, vy): a quarter-warp
-	// (q = 0..7) reads 128 contiguous bytes
-	float4* Vs = reinterpret_cast<float4*>(smem + lay.vs);
-	// c S of the start pair (q * SPT + 2h, +1) of event e at 16-byte chunk
-	// e * SG / 2 + h * NQ + q: again contiguous over q for both phases
+	const BatchSmem lay = batchSmem(W);
+	float2* stages = reinterpret_cast<float2*>(smem + lay.stages);  // [2][W][kBE]
+	float2* Vs = reinterpret_cast<float2*>(smem + lay.vs);          // [W][SG]
+	// c S of starts 2 p and 2 p + 1 of event e at 16-byte slot e * 16 + p
 	float2* Ts = reinterpret_cast<float2*>(smem + lay.ts);          // [2][kBE][SG]
 	float* flat2 = reinterpret_cast<float*>(smem + lay.flat);       // [SG]
 	uint64_t* bars = reinterpret_cast<uint64_t*>(smem + lay.bars);
-	__shared__ double redLL[kBThreads / 32][SG], redC[kBThreads / 32][SG];
+	__shared__ double redLL[8][SG], redC[8][SG];
 
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const uint32_t tileBytes = (uint32_t)W * kBE * 8u;
-	// phase-1 role
-	const int sq = tid % (SG / SPT), eq = tid / (SG / SPT);
-	const int s1 = sq * SPT, e1 = eq * EPT;
-	// phase-2 role
-	const int sp = tid % (SG / SPT2), wg = tid / (SG / SPT2);
-	const int s2 = sp * SPT2, w2 = wg * WPT;
+	const int quad = (lane & 1) | ((lane >> 1) & 6), four = ((lane >> 1) & 1) | ((lane >> 3) & 2);
+	// phase 1: starts 2 p1 and 2 p1 + 1, events 4 (4 (warp mod 8) + four) + 0..3
+	const int p1 = (warp >> 3) * 8 + quad, e1 = 4 * ((warp & 7) * 4 + four);
+	// phase 2: starts 2 p2 and 2 p2 + 1 of waves w2 and w2 + 32 (a wave beyond
+	// the last repeats it, a warp whose second waves all lie beyond leaves them out)
+	const int p2 = (warp & 1) * 8 + quad, w2 = (warp >> 1) * 4 + four;
+	const int nWave = (warp >> 1) * 4 >= W ? 0 : ((warp >> 1) * 4 + 32 >= W ? 1 : 2);
+	uint32_t rowOff[2], rot[2];
+#pragma unroll
+	for (int j = 0; j < 2; ++j) {
+		const int w = min(w2 + 32 * j, W - 1);
+		rowOff[j] = (uint32_t)(w * kBE) * 8u;
+		rot[j] = storeRot((uint32_t)w, kBE) * 8u;
+	}
 
 	if (tid == 0) {
 		mbarInit(&bars[0], 1);
@@ -118,7 +136,7 @@ __global__ void __launch_bounds__(kBThreads, MINB) fdfBatchKernel(const BatchArg
 		if (!__syncthreads_or(act))
 			continue;
 		// production amplitudes of the group's starts
-		for (int k = tid; k < W * SG; k += kBThreads) {
+		for (int k = tid; k < W * SG; k += kB32Threads) {
 			const int w = k / SG, s = k - w * SG;
 			float vr = 0.f, vi = 0.f;
 			if (s < ns) {
@@ -127,17 +145,17 @@ __global__ void __launch_bounds__(kBThreads, MINB) fdfBatchKernel(const BatchArg
 				vr = ir >= 0 ? (float)x[ir] : 0.f;
 				vi = ii >= 0 ? (float)x[ii] : 0.f;
 			}
-			Vs[w * SG + (s % SPT) * NQ + s / SPT] = make_float4(vr, vr, vi, vi);
+			Vs[w * SG + s] = make_float2(vr, vi);
 		}
-		for (int s = tid; s < SG; s += kBThreads) {
-			const double f = (s < ns) ? a.x[(size_t)(q0 + s) * P + P - 1] : 0.;
-			flat2[s] = (float)(f * f);
+		if (tid < SG) {
+			const double f = (tid < ns) ? a.x[(size_t)(q0 + tid) * P + P - 1] : 0.;
+			flat2[tid] = (float)(f * f);
 		}
 		const int nt = (int)(it.t1 - it.t0);
 		const uint32_t ph0[2] = {phase[0], phase[1]};
 		if (tid == 0) {
 			fenceProxyAsync();
-			for (int k = 0; k < NST && k < nt; ++k) {
+			for (int k = 0; k < 2 && k < nt; ++k) {
 				mbarArriveExpectTx(&bars[k], tileBytes);
 				bulkCopyG2S(stages + (size_t)k * W * kBE, bin.amps + (size_t)(it.t0 + k) * W * kBE, tileBytes,
 				            &bars[k]);
@@ -146,81 +164,88 @@ __global__ void __launch_bounds__(kBThreads, MINB) fdfBatchKernel(const BatchArg
 		__syncthreads();
 
 		// accumulators
-		double llD[SPT], csD[SPT];
-		float llF[SPT], csF[SPT], llK[SPT], csK[SPT];  // compensated FP32 sums
+		double llD[2] = {0., 0.}, csD[2] = {0., 0.};
+		float llF[2] = {0.f, 0.f}, csF[2] = {0.f, 0.f}, llK[2] = {0.f, 0.f}, csK[2] = {0.f, 0.f};  // compensated
+		double gD[2][2][2];
+		float2 Pp[2][2], Qp[2][2];  // [start][wave]
 #pragma unroll
-		for (int i = 0; i < SPT; ++i) {
-			llD[i] = csD[i] = 0.;
-			llF[i] = csF[i] = llK[i] = csK[i] = 0.f;
-		}
-		double gD[SPT2][WPT][2];
-		float2 Pp[SPT2][WPT], Qp[SPT2][WPT];
+		for (int i = 0; i < 2; ++i)
 #pragma unroll
-		for (int i = 0; i < SPT2; ++i)
-#pragma unroll
-			for (int j = 0; j < WPT; ++j) {
+			for (int j = 0; j < 2; ++j) {
 				gD[i][j][0] = gD[i][j][1] = 0.;
 				Pp[i][j] = Qp[i][j] = make_float2(0.f, 0.f);
 			}
 
 		int k = 0;
 		for (; k < nt; ++k) {
-			const int st = (NST == 2) ? (k & 1) : 0;
+			const int st = k & 1;
 			const bool ok = mbarWaitBounded(&bars[st], phase[st]);
 			phase[st] ^= 1u;
-			const float2* tile = stages + (size_t)st * W * kBE;
-			const uint32_t tileAddr = smemAddr(tile);
+			const uint32_t tileAddr = smemAddr(stages + (size_t)st * W * kBE);
 			float2* T = Ts + (size_t)(k & 1) * kBE * SG;
 			const uint64_t ev0 = (uint64_t)(it.t0 + k) * kBE;
 
 			// ---- phase 1: S, L, -ln L, c S ----
 			{
-				float2 U[SPT][EPT], Z[SPT][EPT];
+				float2 U[2][4], Z[2][4];
 #pragma unroll
-				for (int i = 0; i < SPT; ++i)
+				for (int i = 0; i < 2; ++i)
 #pragma unroll
-					for (int j = 0; j < EPT; ++j)
+					for (int j = 0; j < 4; ++j)
 						U[i][j] = Z[i][j] = make_float2(0.f, 0.f);
-				const uint32_t vAddr = smemAddr(Vs) + (uint32_t)sq * 16u;
-				for (int w = 0; w < W; ++w) {
-					const int pos = (e1 + (int)storeRot((uint32_t)w, kBE)) & (kBE - 1);
-					float2 av[EPT];
+				auto wave = [&](uint32_t aRow, uint32_t vRow) {
+					const float4 p = lds128(aRow), q = lds128(aRow + 16u);
+					const float2 av[4] = {make_float2(p.x, p.y), make_float2(p.z, p.w), make_float2(q.x, q.y),
+					                      make_float2(q.z, q.w)};
+					const float4 v = lds128(vRow);
 #pragma unroll
-					for (int j = 0; j < EPT; j += 2) {
-						const float4 q = lds128(tileAddr + (uint32_t)(w * kBE + pos + j) * 8u);
-						av[j] = make_float2(q.x, q.y);
-						av[j + 1] = make_float2(q.z, q.w);
-					}
+					for (int i = 0; i < 2; ++i) {
+						const float vr = i ? v.z : v.x, vi = i ? v.w : v.y;
+						const float2 vx = make_float2(vr, vr), vy = make_float2(vi, vi);
 #pragma unroll
-					for (int i = 0; i < SPT; ++i) {
-						const float4 v = lds128(vAddr + (uint32_t)(w * SG + i * NQ) * 16u);
-						const float2 vx = make_float2(v.x, v.y), vy = make_float2(v.z, v.w);
-#pragma unroll
-						for (int j = 0; j < EPT; ++j) {
+						for (int j = 0; j < 4; ++j) {
 							U[i][j] = ffma2(av[j], vx, U[i][j]);
 							Z[i][j] = ffma2(av[j], vy, Z[i][j]);
 						}
 					}
+				};
+				// events 4 g .. 4 g + 3 of wave w: one 32-byte piece at 4 g + rot(w) mod 128
+				uint32_t col[4];
+#pragma unroll
+				for (int r = 0; r < 4; ++r)
+					col[r] = tileAddr + (uint32_t)(r * kBE + ((e1 + (int)storeRot((uint32_t)r, kBE)) & (kBE - 1))) * 8u;
+				uint32_t vAddr = smemAddr(Vs) + (uint32_t)p1 * 16u;
+				int w = 0;
+#pragma unroll 1
+				for (; w + 4 <= W; w += 4) {
+#pragma unroll
+					for (int r = 0; r < 4; ++r)
+						wave(col[r], vAddr + (uint32_t)r * (SG * 8u));
+#pragma unroll
+					for (int r = 0; r < 4; ++r)
+						col[r] += 4u * kBE * 8u;
+					vAddr += 4u * SG * 8u;
 				}
 #pragma unroll
-				for (int j = 0; j < EPT; ++j) {
+				for (int r = 0; r < 3; ++r)
+					if (w + r < W)
+						wave(col[r], vAddr + (uint32_t)r * (SG * 8u));
+#pragma unroll
+				for (int j = 0; j < 4; ++j) {
 					const bool valid = ev0 + (uint64_t)(e1 + j) < bin.nEvents;
+					float2 ts[2];
 #pragma unroll
-					for (int i = 0; i < SPT; i += 2) {
-						float2 ts[2];
-#pragma unroll
-						for (int h = 0; h < 2; ++h) {
-							const float sx = U[i + h][j].x - Z[i + h][j].y, sy = U[i + h][j].y + Z[i + h][j].x;
-							const float L = fmaf(sx, sx, fmaf(sy, sy, flat2[s1 + i + h]));
-							const float c = valid ? -2.f / L : 0.f;
-							if (valid)
-								kahanAdd(llF[i + h], llK[i + h], -logf(L));
-							kahanAdd(csF[i + h], csK[i + h], c);
-							ts[h] = make_float2(c * sx, c * sy);
-						}
-						*reinterpret_cast<float4*>(&T[2 * ((e1 + j) * (SG / 2) + (i / 2) * NQ + sq)]) =
-						    make_float4(ts[0].x, ts[0].y, ts[1].x, ts[1].y);
+					for (int i = 0; i < 2; ++i) {
+						const float sx = U[i][j].x - Z[i][j].y, sy = U[i][j].y + Z[i][j].x;
+						const float L = fmaf(sx, sx, fmaf(sy, sy, flat2[2 * p1 + i]));
+						const float c = valid ? -2.f / L : 0.f;
+						if (valid)
+							kahanAdd(llF[i], llK[i], -logf(L));
+						kahanAdd(csF[i], csK[i], c);
+						ts[i] = make_float2(c * sx, c * sy);
 					}
+					*reinterpret_cast<float4*>(&T[2 * ((e1 + j) * 16 + p1)]) =
+					    make_float4(ts[0].x, ts[0].y, ts[1].x, ts[1].y);
 				}
 			}
 			// T complete; phase 2 of the previous tile is done by every thread
@@ -228,7 +253,7 @@ __global__ void __launch_bounds__(kBThreads, MINB) fdfBatchKernel(const BatchArg
 				failed = true;
 				break;
 			}
-			if (NST == 2 && tid == 0 && k >= 1 && k + 1 < nt) {
+			if (tid == 0 && k >= 1 && k + 1 < nt) {
 				fenceProxyAsync();
 				const int ns2 = (k + 1) & 1;
 				mbarArriveExpectTx(&bars[ns2], tileBytes);
@@ -237,54 +262,53 @@ __global__ void __launch_bounds__(kBThreads, MINB) fdfBatchKernel(const BatchArg
 			}
 
 			// ---- phase 2: G += sum_e c S conj(A) ----
-			if (w2 < W) {
-				const uint32_t tAddr = smemAddr(T) + (uint32_t)sp * 16u;
-				int rot[WPT];
+			auto sums = [&](auto nw) {
+				constexpr int NW = decltype(nw)::value;
+				uint32_t tAddr = smemAddr(T) + (uint32_t)p2 * 16u;
+#pragma unroll 1
+				for (uint32_t e = 0; e < (uint32_t)kBE * 8u; e += 32u, tAddr += 4u * SG * 8u) {
+					float2 av[NW][4];
 #pragma unroll
-				for (int j = 0; j < WPT; ++j)
-					rot[j] = (int)storeRot((uint32_t)(w2 + j), kBE);
-				for (int e = 0; e < kBE; ++e) {
-					float2 t[SPT2];
-#pragma unroll
-					for (int i = 0; i < SPT2; i += 2) {
-						const float4 q = lds128(tAddr + (uint32_t)(e * (SG / 2) + (i / 2) * NQ) * 16u);
-						t[i] = make_float2(q.x, q.y);
-						t[i + 1] = make_float2(q.z, q.w);
+					for (int j = 0; j < NW; ++j) {
+						const uint32_t pos = tileAddr + rowOff[j] + ((e + rot[j]) & (kBE * 8u - 1u));
+						const float4 p = lds128(pos), q = lds128(pos + 16u);
+						av[j][0] = make_float2(p.x, p.y);
+						av[j][1] = make_float2(p.z, p.w);
+						av[j][2] = make_float2(q.x, q.y);
+						av[j][3] = make_float2(q.z, q.w);
 					}
 #pragma unroll
-					for (int j = 0; j < WPT; ++j) {
-						const int w = min(w2 + j, W - 1);
-						const float2 av = lds64(tileAddr + (uint32_t)(w * kBE + ((e + rot[j]) & (kBE - 1))) * 8u);
-						const float2 aw = make_float2(av.y, av.x);
+					for (int x = 0; x < 4; ++x) {
+						const float4 tt = lds128(tAddr + (uint32_t)x * (SG * 8u));
+						const float2 t[2] = {make_float2(tt.x, tt.y), make_float2(tt.z, tt.w)};
 #pragma unroll
-						for (int i = 0; i < SPT2; ++i) {
-							Pp[i][j] = ffma2(t[i], av, Pp[i][j]);  // (tx ax, ty ay)
-							Qp[i][j] = ffma2(t[i], aw, Qp[i][j]);  // (tx ay, ty ax)
+						for (int j = 0; j < NW; ++j) {
+							const float2 aw = make_float2(av[j][x].y, av[j][x].x);
+#pragma unroll
+							for (int i = 0; i < 2; ++i) {
+								Pp[i][j] = ffma2(t[i], av[j][x], Pp[i][j]);  // (tx ax, ty ay)
+								Qp[i][j] = ffma2(t[i], aw, Qp[i][j]);        // (tx ay, ty ax)
+							}
 						}
 					}
 				}
-			}
-			// one stage: the next tile loads once every thread is done with this one
-			if (NST == 1) {
-				__syncthreads();
-				if (tid == 0 && k + 1 < nt) {
-					fenceProxyAsync();
-					mbarArriveExpectTx(&bars[0], tileBytes);
-					bulkCopyG2S(stages, bin.amps + (size_t)(it.t0 + k + 1) * W * kBE, tileBytes, &bars[0]);
-				}
-			}
+			};
+			if (nWave == 2)
+				sums(std::integral_constant<int, 2>{});
+			else if (nWave == 1)
+				sums(std::integral_constant<int, 1>{});
 			// fold the FP32 partials into FP64
 			if ((k + 1) % kBFold == 0 || k + 1 == nt) {
 #pragma unroll
-				for (int i = 0; i < SPT; ++i) {
+				for (int i = 0; i < 2; ++i) {
 					llD[i] += (double)llF[i] - (double)llK[i];
 					csD[i] += (double)csF[i] - (double)csK[i];
 					llF[i] = csF[i] = llK[i] = csK[i] = 0.f;
 				}
 #pragma unroll
-				for (int i = 0; i < SPT2; ++i)
+				for (int i = 0; i < 2; ++i)
 #pragma unroll
-					for (int j = 0; j < WPT; ++j) {
+					for (int j = 0; j < 2; ++j) {
 						gD[i][j][0] += (double)(Pp[i][j].x + Pp[i][j].y);
 						gD[i][j][1] += (double)(Qp[i][j].y - Qp[i][j].x);
 						Pp[i][j] = Qp[i][j] = make_float2(0.f, 0.f);
@@ -295,14 +319,9 @@ __global__ void __launch_bounds__(kBThreads, MINB) fdfBatchKernel(const BatchArg
 			if (tid == 0) {
 				atomicOr(a.devErr, (unsigned)kDevErrTimeout);
 				// copies of this item still in flight land before the block
-				// exits: with two stages tiles k .. max(1, k) were issued and
-				// not consumed, with one stage tile k
-				if (NST == 2) {
-					for (int j = k; j <= max(1, k) && j < nt; ++j)
-						mbarWaitBounded(&bars[j & 1], ph0[j & 1] ^ (uint32_t)((j >> 1) & 1));
-				} else if (k < nt) {
-					mbarWaitBounded(&bars[0], ph0[0] ^ (uint32_t)(k & 1));
-				}
+				// exits: tiles k .. max(1, k) were issued and not consumed
+				for (int j = k; j <= max(1, k) && j < nt; ++j)
+					mbarWaitBounded(&bars[j & 1], ph0[j & 1] ^ (uint32_t)((j >> 1) & 1));
 			}
 			break;
 		}
@@ -310,38 +329,37 @@ __global__ void __launch_bounds__(kBThreads, MINB) fdfBatchKernel(const BatchArg
 		// ---- partials of this item: [SG][2 + 2W] FP64 ----
 		const int NV = 2 + 2 * W;
 		double* out = a.partials + (size_t)item * SG * NV;
-		// LL and sum c per start: lanes that share sq differ in eq
+		// LL and sum c per start, over the warp's four event groups
 #pragma unroll
-		for (int i = 0; i < SPT; ++i) {
+		for (int i = 0; i < 2; ++i) {
 			double l = llD[i], c = csD[i];
-			for (int o = SG / SPT; o < 32; o <<= 1) {
-				l += __shfl_xor_sync(0xffffffffu, l, o);
-				c += __shfl_xor_sync(0xffffffffu, c, o);
-			}
-			if (lane < SG / SPT) {
-				redLL[warp][s1 + i] = l;
-				redC[warp][s1 + i] = c;
+			l += __shfl_xor_sync(0xffffffffu, l, 2);
+			c += __shfl_xor_sync(0xffffffffu, c, 2);
+			l += __shfl_xor_sync(0xffffffffu, l, 16);
+			c += __shfl_xor_sync(0xffffffffu, c, 16);
+			if (four == 0) {
+				redLL[warp & 7][2 * p1 + i] = l;
+				redC[warp & 7][2 * p1 + i] = c;
 			}
 		}
-		if (w2 < W) {
 #pragma unroll
-			for (int i = 0; i < SPT2; ++i)
+		for (int i = 0; i < 2; ++i)
 #pragma unroll
-				for (int j = 0; j < WPT; ++j)
-					if (w2 + j < W) {
-						out[(size_t)(s2 + i) * NV + 2 + 2 * (w2 + j)] = gD[i][j][0];
-						out[(size_t)(s2 + i) * NV + 3 + 2 * (w2 + j)] = gD[i][j][1];
-					}
-		}
+			for (int j = 0; j < 2; ++j)
+				if (w2 + 32 * j < W) {
+					double* o = out + (size_t)(2 * p2 + i) * NV + 2 + 2 * (w2 + 32 * j);
+					o[0] = gD[i][j][0];
+					o[1] = gD[i][j][1];
+				}
 		__syncthreads();
-		for (int s = tid; s < SG; s += kBThreads) {
+		if (tid < SG) {
 			double l = 0., c = 0.;
-			for (int wv = 0; wv < kBThreads / 32; ++wv) {
-				l += redLL[wv][s];
-				c += redC[wv][s];
+			for (int wv = 0; wv < 8; ++wv) {
+				l += redLL[wv][tid];
+				c += redC[wv][tid];
 			}
-			out[(size_t)s * NV] = l;
-			out[(size_t)s * NV + 1] = c;
+			out[(size_t)tid * NV] = l;
+			out[(size_t)tid * NV + 1] = c;
 		}
 		__syncthreads();
 	}
@@ -980,33 +998,6 @@ __global__ void countActiveKernel(const int* status, int Q, int* active, unsigne
 	}
 }
 
-template <int SG, int SPT, int EPT, int SPT2, int WPT, int NST, int MINB>
-int configureBatchT(int W)
-{
-	const BatchSmem lay = batchSmem(W, SG, NST);
-	return cudaCheck(cudaFuncSetAttribute(fdfBatchKernel<SG, SPT, EPT, SPT2, WPT, NST, MINB>,
-	                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.total),
-	                 "batch smem attribute");
-}
-
-// persistent grid: numSMs x the blocks of this variant that fit on an SM
-template <int SG, int SPT, int EPT, int SPT2, int WPT, int NST, int MINB>
-int launchBatchT(const BatchArgs& a, int numSMs, cudaStream_t s)
-{
-	auto kern = fdfBatchKernel<SG, SPT, EPT, SPT2, WPT, NST, MINB>;
-	const BatchSmem lay = batchSmem(a.W, SG, NST);
-	int perSM = 1;
-	if (NST == 1) {
-		const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, kBThreads, lay.total);
-		if (e != cudaSuccess)
-			return cudaCheck(e, "batch FdF occupancy");
-		perSM = std::max(1, std::min(perSM, MINB));
-	}
-	kern<<<numSMs * perSM, kBThreads, lay.total, s>>>(a);
-	countLaunches(1);
-	return cudaCheck(cudaGetLastError(), "batch FdF launch");
-}
-
 // persistent grid: numSMs x the blocks that fit on an SM (at most three)
 int launchBatch8(const BatchArgs& a, int numSMs, cudaStream_t s)
 {
@@ -1023,7 +1014,7 @@ int launchBatch8(const BatchArgs& a, int numSMs, cudaStream_t s)
 
 }  // namespace
 
-size_t batchSmemBytes(int W, int SG) { return SG == 8 ? batch8Smem(W).total : batchSmem(W, SG, 2).total; }
+size_t batchSmemBytes(int W, int SG) { return SG == 8 ? batch8Smem(W).total : batchSmem(W).total; }
 
 // start groups of 32: two stages, one block per SM; of 8: the
 // register-blocked kernel, one stage, up to three blocks per SM
@@ -1034,7 +1025,9 @@ int configureBatchFdf(int W, int SG, size_t maxSmem)
 	if (batchSmemBytes(W, SG) > maxSmem)
 		return setError(kErrUnsupported, "batched FdF: shared memory too small for this wave set");
 	if (SG == 32)
-		return configureBatchT<32, 4, 4, 4, 2, 2, 1>(W);
+		return cudaCheck(cudaFuncSetAttribute(fdfBatch32Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                                      (int)batchSmem(W).total),
+		                 "batch smem attribute");
 	if (SG == 8)
 		return cudaCheck(cudaFuncSetAttribute(fdfBatch8Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		                                      (int)batch8Smem(W).total),
@@ -1046,8 +1039,11 @@ int launchBatchFdf(const BatchArgs& a, int numSMs, cudaStream_t s)
 {
 	if (a.W < 1 || a.W > 64)
 		return setError(kErrUnsupported, "batched FdF supports 1..64 waves");
-	if (a.SG == 32)
-		return launchBatchT<32, 4, 4, 4, 2, 2, 1>(a, numSMs, s);
+	if (a.SG == 32) {
+		fdfBatch32Kernel<<<numSMs, kB32Threads, batchSmem(a.W).total, s>>>(a);
+		countLaunches(1);
+		return cudaCheck(cudaGetLastError(), "batch FdF launch");
+	}
 	if (a.SG == 8)
 		return launchBatch8(a, numSMs, s);
 	return setError(kErrUnsupported, "batched FdF: start-group size must be 8 or 32");
