@@ -23,8 +23,8 @@
 //                       tile): register-blocked phases over a quarter of the
 //                       waves or events per thread, combined by shuffles; one
 //                       stage, several blocks per SM taking turns;
-//   batchFinishKernel -- one warp per problem: sums the items' partials in item
-//                       order (deterministic), adds nEvt (Re V^H I^acc V +
+//   batchFinishKernel -- half a block per problem: sums the items' partials in
+//                       item order (deterministic), adds nEvt (Re V^H I^acc V +
 //                       V_flat^2 eta) and the half-Cauchy prior in FP64
 //                       (pwaLikelihood.cc:254-297) and writes f and the gradient;
 //   lbfgsKernel      -- one warp per problem: backtracking line search
@@ -687,86 +687,121 @@ __device__ __forceinline__ double warpAllSum(double v)
 	return v;
 }
 
-// One warp per problem: f and gradient from the items' partials plus the
-// normalisation and prior terms.
-__global__ void batchFinishKernel(const FinishBatchArgs a)
+// f and gradient from the items' partials plus the normalisation and prior
+// terms, two problems per block.  Four warps form a problem's rows
+//   D_i = sum_j V_j conj(I_ij)
+// (64 threads per problem, one row each: the FP64 pipe's work) while the other
+// four add up the items' partials, one value per thread with eight loads in
+// flight.  With one warp per problem the serial loads of both bounded it: 92 us
+// for 512 problems of 50 waves and 8 to 79 items, 27 now; 117 us for 1536,
+// 83 now (the FP64 pipe then).
+constexpr int kFinProblems = 2, kFinThreads = 256, kFinWaves = 64;
+__global__ void __launch_bounds__(kFinThreads) batchFinishKernel(const FinishBatchArgs a)
 {
-	const int q = (int)((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5);
-	const int lane = threadIdx.x & 31;
-	if (q >= a.Q || !a.active[q])
-		return;
+	__shared__ double ev[kFinProblems][2 + 2 * kFinWaves];  // event sums
+	__shared__ double2 vs[kFinProblems][kFinWaves];
+	__shared__ double tn[kFinProblems][kFinWaves], tp[kFinProblems][kFinWaves];
+	const int tid = threadIdx.x, lane = tid & 31;
 	const int W = a.W, P = a.P, NV = 2 + 2 * W;
-	const ProblemDesc pd = a.problems[q];
-	const BinDesc bin = a.bins[pd.bin];
+	const int q0 = (int)blockIdx.x * kFinProblems;
+	const int pl = (tid >> 6) & 1, i = tid & 63;  // warps 0..3: problem and row
+	const int q = q0 + pl;
+	const bool act = q < a.Q && a.active[q];
 	const double* x = a.x + (size_t)q * P;
-	double* g = a.g + (size_t)q * P;
-	const double nEvt = bin.nEvt, twice = 2. * bin.nEvt;
-	const double flat = x[P - 1];
-	// event sums, in item order
-	double fLL = 0., fC = 0.;
-	for (int v = lane; v < NV; v += 32) {
-		double acc = 0.;
-		for (int i = pd.item0; i < pd.item1; ++i)
-			acc += a.partials[((size_t)i * a.SG + pd.slot) * NV + v];
-		if (v == 0)
-			fLL = acc;
-		else if (v == 1)
-			fC = acc;
-		else {
-			const int w = (v - 2) >> 1, comp = (v - 2) & 1;
-			const int idx = comp ? a.slotIm[w] : a.slotRe[w];
-			if (idx >= 0)
-				g[idx] = acc;
+	ProblemDesc pd{};
+	BinDesc bin{};
+	if (act) {
+		pd = a.problems[q];
+		bin = a.bins[pd.bin];
+	}
+	const bool rows = tid < 64 * kFinProblems;
+	int ri = -1, ii = -1;
+	double vr = 0., vi = 0.;
+	if (rows && act && i < W) {
+		ri = a.slotRe[i];
+		ii = a.slotIm[i];
+		vr = ri >= 0 ? x[ri] : 0.;
+		vi = ii >= 0 ? x[ii] : 0.;
+		vs[pl][i] = make_double2(vr, vi);
+	}
+	__syncthreads();
+	const double twice = 2. * bin.nEvt;
+	double dre = 0., dim = 0., pre = 0., pim = 0.;
+	if (rows) {
+		if (act && i < W) {
+			const double2* Ib = reinterpret_cast<const double2*>(bin.accI) + (size_t)i * W;
+#pragma unroll 4
+			for (int j = 0; j < W; ++j) {
+				const double2 u = vs[pl][j], I = __ldg(Ib + j);
+				const double ur = u.x, ui = u.y, Ir = I.x, Ii = I.y;
+				dre += ur * Ir + ui * Ii;
+				dim += ui * Ir - ur * Ii;
+			}
+			double prior = 0.;
+			if (a.prior == 1) {
+				const double g2 = a.cauchyWidth * a.cauchyWidth;
+				const double rr = hypot(vr, vi);
+				const double cf = 1. / (1. + (rr * rr) / g2);
+				const double cd = (-2. * rr * g2) / ((g2 + rr * rr) * (g2 + rr * rr));
+				const double fac = (1. / (rr * cf)) * cd;
+				prior = -log(cf);
+				pre = fac * vr;
+				pim = fac * vi;
+			}
+			tn[pl][i] = __fma_rn(vr, dre, __dmul_rn(vi, dim));
+			tp[pl][i] = prior;
+		}
+	} else {
+		// event sums, in item order
+		for (int t = tid - 64 * kFinProblems; t < kFinProblems * NV; t += kFinThreads - 64 * kFinProblems) {
+			const int p = t >= NV ? 1 : 0, v = t - p * NV;
+			if (q0 + p >= a.Q || !a.active[q0 + p])
+				continue;
+			const ProblemDesc d = a.problems[q0 + p];
+			const size_t step = (size_t)a.SG * NV;
+			const double* src = a.partials + (size_t)d.item0 * step + (size_t)d.slot * NV + v;
+			double acc = 0.;
+			int n = d.item1 - d.item0;
+			for (; n >= 8; n -= 8, src += 8 * step) {
+				double c[8];
+#pragma unroll
+				for (int k = 0; k < 8; ++k)
+					c[k] = src[k * step];
+#pragma unroll
+				for (int k = 0; k < 8; ++k)
+					acc += c[k];
+			}
+			for (; n > 0; --n, src += step)
+				acc += *src;
+			ev[p][v] = acc;
 		}
 	}
-	fLL = __shfl_sync(0xffffffffu, fLL, 0);
-	fC = __shfl_sync(0xffffffffu, fC, 1);
-	__syncwarp();
-	// normalisation: D_i = sum_j V_j conj(I_ij); prior
-	double norm = 0., prior = 0.;
-	const double g2 = a.cauchyWidth * a.cauchyWidth;
-	for (int i = lane; i < W; i += 32) {
-		const int ri = a.slotRe[i], ii = a.slotIm[i];
-		const double vr = ri >= 0 ? x[ri] : 0., vi = ii >= 0 ? x[ii] : 0.;
-		double dre = 0., dim = 0.;
-		const double* Ib = bin.accI + (size_t)2 * i * W;
-		for (int j = 0; j < W; ++j) {
-			const int rj = a.slotRe[j], ij = a.slotIm[j];
-			const double ur = rj >= 0 ? x[rj] : 0., ui = ij >= 0 ? x[ij] : 0.;
-			const double Ir = Ib[2 * j], Ii = Ib[2 * j + 1];
-			dre += ur * Ir + ui * Ii;
-			dim += ui * Ir - ur * Ii;
-		}
-		norm += vr * dre + vi * dim;
-		double pre = 0., pim = 0.;
-		if (a.prior == 1) {
-			const double rr = hypot(vr, vi);
-			const double cf = 1. / (1. + (rr * rr) / g2);
-			const double cd = (-2. * rr * g2) / ((g2 + rr * rr) * (g2 + rr * rr));
-			const double fac = (1. / (rr * cf)) * cd;
-			prior += -log(cf);
-			pre = fac * vr;
-			pim = fac * vi;
-		}
-		if (ri >= 0)
-			g[ri] += twice * dre - pre;
-		if (ii >= 0)
-			g[ii] += twice * dim - pim;
-	}
-	norm = warpAllSum(norm);
-	prior = warpAllSum(prior);
-	if (lane == 0) {
-		a.f[q] = fLL + nEvt * (norm + flat * flat * bin.totAcc) + prior;
-		g[P - 1] = flat * fC + twice * flat * bin.totAcc;
-	}
+	__syncthreads();
+	if (!rows || !act)
+		return;
 	// parameters the layout holds fixed do not move: their gradient
 	// components are 0 to the minimiser (the reference strips them,
 	// highLevelInterface/pwaNloptFit.cc:383-401)
-	__syncwarp();
+	double* g = a.g + (size_t)q * P;
 	const unsigned char* fx = a.fixed + (size_t)pd.bin * P;
-	for (int i = lane; i < P; i += 32)
-		if (fx[i])
-			g[i] = 0.;
+	if (ri >= 0)
+		g[ri] = fx[ri] ? 0. : ev[pl][2 + 2 * i] + (twice * dre - pre);
+	if (ii >= 0)
+		g[ii] = fx[ii] ? 0. : ev[pl][3 + 2 * i] + (twice * dim - pim);
+	if (i < 32) {
+		double norm = 0., prior = 0.;
+		for (int k = lane; k < W; k += 32) {
+			norm += tn[pl][k];
+			prior += tp[pl][k];
+		}
+		norm = warpAllSum(norm);
+		prior = warpAllSum(prior);
+		if (lane == 0) {
+			const double nEvt = bin.nEvt, flat = x[P - 1];
+			a.f[q] = ev[pl][0] + nEvt * (norm + flat * flat * bin.totAcc) + prior;
+			g[P - 1] = fx[P - 1] ? 0. : flat * ev[pl][1] + twice * flat * bin.totAcc;
+		}
+	}
 }
 
 // General-layout batches: problem q's FdF launch wrote [f, gradient, device
@@ -794,33 +829,63 @@ __global__ void gatherEvalKernel(const GatherEvalArgs a)
 // ---------------------------------------------------------------------------
 // batched L-BFGS (one warp per problem, FP64)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double wdot(const double* a, const double* b, int n, int lane)
+// NE > 0: the vectors (P <= 32 NE) live in registers, element lane + 32 k in
+// [k], and the next history pair loads while one is used; NE = 0: any P, the
+// vectors stay in memory.  Same sums in the same order.  What bounds it is the
+// chain of 2 x history length warp sums; with the vectors in memory every one
+// of them waited for L2 (71 us per sweep of 512 problems of 100 parameters and
+// eight history pairs, 26 now).
+template <int NE>
+__global__ void __launch_bounds__(32) lbfgsKernel(const LbfgsArgs a)
 {
-	double s = 0.;
-	for (int i = lane; i < n; i += 32)
-		s += a[i] * b[i];
-	return warpAllSum(s);
-}
-
-__global__ void lbfgsKernel(const LbfgsArgs a)
-{
-	const int q = (int)((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5);
-	const int lane = threadIdx.x & 31;
-	if (q >= a.Q)
-		return;
+	constexpr int R = NE > 0 ? NE : 1;
+	const int q = (int)blockIdx.x;
+	const int lane = threadIdx.x;
 	const int st = a.status[q];
 	if (st != kLbfgsInit && st != kLbfgsSearch)
 		return;
 	const int P = a.P, m = a.m;
-	double* x = a.x + (size_t)q * P;    // accepted point
-	double* g = a.g + (size_t)q * P;
-	double* d = a.d + (size_t)q * P;
-	double* xt = a.xt + (size_t)q * P;  // trial point (evaluated in this sweep)
-	const double* gt = a.gt + (size_t)q * P;
+	double* const x = a.x + (size_t)q * P;    // accepted point
+	double* const g = a.g + (size_t)q * P;
+	double* const d = a.d + (size_t)q * P;
+	double* const xt = a.xt + (size_t)q * P;  // trial point (evaluated in this sweep)
+	const double* const gt = a.gt + (size_t)q * P;
 	double* S = a.S + (size_t)q * m * P;
 	double* Y = a.Y + (size_t)q * m * P;
 	double* rho = a.rho + (size_t)q * m;
 	double* alph = a.alphaBuf + (size_t)q * m;
+	// f(i, k) for this lane's elements i
+	auto each = [&](auto f) {
+		if constexpr (NE > 0) {
+#pragma unroll
+			for (int k = 0; k < NE; ++k)
+				if (lane + 32 * k < P)
+					f(lane + 32 * k, k);
+		} else {
+			for (int i = lane; i < P; i += 32)
+				f(i, 0);
+		}
+	};
+	double rx[R], rg[R], rd[R], rxt[R], rgt[R];
+	if constexpr (NE > 0)
+		each([&](int i, int k) {
+			rx[k] = x[i];
+			rg[k] = g[i];
+			rd[k] = d[i];
+			rxt[k] = xt[i];
+			rgt[k] = gt[i];
+		});
+	// element i of a vector: its register or its place in memory
+	auto X = [&](int i, int k) -> double& { return NE > 0 ? rx[k] : x[i]; };
+	auto G = [&](int i, int k) -> double& { return NE > 0 ? rg[k] : g[i]; };
+	auto D = [&](int i, int k) -> double& { return NE > 0 ? rd[k] : d[i]; };
+	auto XT = [&](int i, int k) -> double& { return NE > 0 ? rxt[k] : xt[i]; };
+	auto GT = [&](int i, int k) -> double { return NE > 0 ? rgt[k] : gt[i]; };
+	auto dot = [&](auto u, auto v) {
+		double s = 0.;
+		each([&](int i, int k) { s += u(i, k) * v(i, k); });
+		return warpAllSum(s);
+	};
 	const double ft = a.ft[q];
 	bool accept = false;
 	if (st == kLbfgsInit) {
@@ -835,8 +900,8 @@ __global__ void lbfgsKernel(const LbfgsArgs a)
 		// Hager and Zhang (value within a relative 1e-8 of f, directional
 		// derivative between 0.9 g.d and -0.8 g.d), which stay decisive when
 		// the decrease is below the rounding noise of f near a minimum
-		const double gd = wdot(g, d, P, lane);
-		const double gtd = wdot(gt, d, P, lane);
+		const double gd = dot(G, D);
+		const double gtd = dot(GT, D);
 		const double f0 = a.f[q];
 		const bool armijo = ft <= f0 + 1e-4 * a.step[q] * gd;
 		const bool approxWolfe = ft <= f0 + 1e-8 * fmax(1., fabs(f0)) && gtd >= 0.9 * gd && gtd <= -0.8 * gd;
@@ -849,11 +914,12 @@ __global__ void lbfgsKernel(const LbfgsArgs a)
 		if (nb > 40) {
 			if (a.hist[q] > 0) {
 				// restart once from steepest descent at the accepted point
-				const double gn = sqrt(wdot(g, g, P, lane));
-				for (int i = lane; i < P; i += 32) {
-					d[i] = -g[i] / fmax(gn, 1e-300);
-					xt[i] = x[i] + d[i];
-				}
+				const double gn = sqrt(dot(G, G));
+				each([&](int i, int k) {
+					const double di = -G(i, k) / fmax(gn, 1e-300);
+					d[i] = di;
+					xt[i] = X(i, k) + di;
+				});
 				if (lane == 0) {
 					a.hist[q] = 0;
 					a.head[q] = 0;
@@ -866,8 +932,7 @@ __global__ void lbfgsKernel(const LbfgsArgs a)
 				a.status[q] = kLbfgsStalled;
 			return;
 		}
-		for (int i = lane; i < P; i += 32)
-			xt[i] = x[i] + step * d[i];
+		each([&](int i, int k) { xt[i] = X(i, k) + step * D(i, k); });
 		if (lane == 0) {
 			a.nBack[q] = nb;
 			a.step[q] = step;
@@ -876,26 +941,31 @@ __global__ void lbfgsKernel(const LbfgsArgs a)
 	}
 	// accept the trial point: update the history with s = xt - x, y = gt - g
 	int hist = a.hist[q], head = a.head[q];
+	double gamma = hist > 0 ? a.gamma[q] : 0.;
+	double rhoNew = 0.;
+	int slotNew = -1;
 	if (st == kLbfgsSearch) {
 		double sy = 0., yy = 0., ss = 0.;
-		for (int i = lane; i < P; i += 32) {
-			const double si = xt[i] - x[i], yi = gt[i] - g[i];
+		each([&](int i, int k) {
+			const double si = XT(i, k) - X(i, k), yi = GT(i, k) - G(i, k);
 			sy += si * yi;
 			yy += yi * yi;
 			ss += si * si;
-		}
+		});
 		sy = warpAllSum(sy);
 		yy = warpAllSum(yy);
 		ss = warpAllSum(ss);
 		if (sy > 1e-12 * sqrt(ss * yy)) {
-			const int slot = (head + hist) % m;
-			for (int i = lane; i < P; i += 32) {
-				S[(size_t)slot * P + i] = xt[i] - x[i];
-				Y[(size_t)slot * P + i] = gt[i] - g[i];
-			}
+			slotNew = (head + hist) % m;
+			each([&](int i, int k) {
+				S[(size_t)slotNew * P + i] = XT(i, k) - X(i, k);
+				Y[(size_t)slotNew * P + i] = GT(i, k) - G(i, k);
+			});
+			rhoNew = 1. / sy;
+			gamma = sy / yy;
 			if (lane == 0) {
-				rho[slot] = 1. / sy;
-				a.gamma[q] = sy / yy;
+				rho[slotNew] = rhoNew;
+				a.gamma[q] = gamma;
 			}
 			if (hist < m)
 				++hist;
@@ -904,13 +974,17 @@ __global__ void lbfgsKernel(const LbfgsArgs a)
 		}
 	}
 	__syncwarp();
-	for (int i = lane; i < P; i += 32) {
-		x[i] = xt[i];
-		g[i] = gt[i];
-	}
+	each([&](int i, int k) {
+		if constexpr (NE > 0) {
+			rx[k] = rxt[k];
+			rg[k] = rgt[k];
+		}
+		x[i] = XT(i, k);
+		g[i] = GT(i, k);
+	});
 	__syncwarp();
 	const double fNew = ft;
-	const double gnorm = sqrt(wdot(g, g, P, lane));
+	const double gnorm = sqrt(dot(G, G));
 	const int iter = a.iter[q] + (st == kLbfgsSearch ? 1 : 0);
 	if (lane == 0) {
 		a.f[q] = fNew;
@@ -944,43 +1018,89 @@ __global__ void lbfgsKernel(const LbfgsArgs a)
 		return;
 	}
 	// two-loop recursion: d = -H g
-	for (int i = lane; i < P; i += 32)
-		d[i] = -g[i];
+	each([&](int i, int k) { D(i, k) = -G(i, k); });
 	__syncwarp();
-	for (int k = hist - 1; k >= 0; --k) {
+	// pair k of the history: 1 / s.y and, in registers, s and y
+	double sv[2][R], yv[2][R], rv[2];
+	auto load = [&](int k, int b) {
 		const int slot = (head + k) % m;
-		const double al = rho[slot] * wdot(S + (size_t)slot * P, d, P, lane);
+		rv[b] = slot == slotNew ? rhoNew : rho[slot];
+		if constexpr (NE > 0)
+			each([&](int i, int e) {
+				sv[b][e] = S[(size_t)slot * P + i];
+				yv[b][e] = Y[(size_t)slot * P + i];
+			});
+	};
+	// element i of the loaded pair
+	auto SV = [&](int b, size_t o, int i, int e) {
+		if constexpr (NE > 0)
+			return sv[b][e];
+		else
+			return S[o + i];
+	};
+	auto YV = [&](int b, size_t o, int i, int e) {
+		if constexpr (NE > 0)
+			return yv[b][e];
+		else
+			return Y[o + i];
+	};
+	double alphaLane = 0.;  // pair `lane`'s coefficient (history of up to 32 pairs)
+	auto descend = [&](int k, int b) {
+		const size_t o = (size_t)((head + k) % m) * P;
+		if (k > 0)
+			load(k - 1, b ^ 1);
+		const double al = rv[b] * dot([&](int i, int e) { return SV(b, o, i, e); }, D);
 		if (lane == 0)
 			alph[k] = al;
-		for (int i = lane; i < P; i += 32)
-			d[i] -= al * Y[(size_t)slot * P + i];
+		if (lane == k)
+			alphaLane = al;
+		each([&](int i, int e) { D(i, e) -= al * YV(b, o, i, e); });
 		__syncwarp();
+	};
+	auto ascend = [&](int k, int b) {
+		const size_t o = (size_t)((head + k) % m) * P;
+		if (k + 1 < hist)
+			load(k + 1, b ^ 1);
+		const double be = __dmul_rn(rv[b], dot([&](int i, int e) { return YV(b, o, i, e); }, D));
+		const double al = m <= 32 ? __shfl_sync(0xffffffffu, alphaLane, k & 31)
+		                          : __shfl_sync(0xffffffffu, lane == 0 ? alph[k] : 0., 0);
+		each([&](int i, int e) { D(i, e) += (al - be) * SV(b, o, i, e); });
+		__syncwarp();
+	};
+	if (hist > 0)
+		load(hist - 1, 0);
+	for (int k = hist - 1; k >= 0; k -= 2) {
+		descend(k, 0);
+		if (k > 0)
+			descend(k - 1, 1);
 	}
-	const double gamma = hist > 0 ? a.gamma[q] : 1. / fmax(gnorm, 1e-300);
-	for (int i = lane; i < P; i += 32)
-		d[i] *= gamma;
+	const double scale = hist > 0 ? gamma : 1. / fmax(gnorm, 1e-300);
+	// (products rounded here and below, not fused into the sums that follow: a
+	// fit's path does not depend on the kernel's form)
+	each([&](int i, int k) { D(i, k) = __dmul_rn(D(i, k), scale); });
 	__syncwarp();
-	for (int k = 0; k < hist; ++k) {
-		const int slot = (head + k) % m;
-		const double be = rho[slot] * wdot(Y + (size_t)slot * P, d, P, lane);
-		const double al = __shfl_sync(0xffffffffu, lane == 0 ? alph[k] : 0., 0);
-		for (int i = lane; i < P; i += 32)
-			d[i] += (al - be) * S[(size_t)slot * P + i];
-		__syncwarp();
+	if (hist > 0)
+		load(0, 0);
+	for (int k = 0; k < hist; k += 2) {
+		ascend(k, 0);
+		if (k + 1 < hist)
+			ascend(k + 1, 1);
 	}
-	const double gd = wdot(g, d, P, lane);
+	const double gd = dot(G, D);
 	if (!(gd < 0.)) {
 		// not a descent direction: restart from steepest descent
-		for (int i = lane; i < P; i += 32)
-			d[i] = -g[i] / fmax(gnorm, 1e-300);
+		each([&](int i, int k) { D(i, k) = -G(i, k) / fmax(gnorm, 1e-300); });
 		if (lane == 0) {
 			a.hist[q] = 0;
 			a.head[q] = 0;
 		}
 		__syncwarp();
 	}
-	for (int i = lane; i < P; i += 32)
-		xt[i] = x[i] + d[i];
+	each([&](int i, int k) {
+		if constexpr (NE > 0)
+			d[i] = rd[k];
+		xt[i] = X(i, k) + D(i, k);
+	});
 	if (lane == 0) {
 		a.step[q] = 1.;
 		a.nBack[q] = 0;
@@ -1051,9 +1171,11 @@ int launchBatchFdf(const BatchArgs& a, int numSMs, cudaStream_t s)
 
 int launchBatchFinish(const FinishBatchArgs& a, cudaStream_t s)
 {
-	const int threads = 256;
-	const int blocks = (int)((a.Q * 32ull + threads - 1) / threads);
-	batchFinishKernel<<<std::max(blocks, 1), threads, 0, s>>>(a);
+	static_assert(kFinProblems == 2, "the item sums' split");
+	if (a.W < 1 || a.W > kFinWaves)
+		return setError(kErrUnsupported, "batched FdF supports 1..64 waves");
+	const int blocks = (a.Q + kFinProblems - 1) / kFinProblems;
+	batchFinishKernel<<<std::max(blocks, 1), kFinThreads, 0, s>>>(a);
 	countLaunches(1);
 	return cudaCheck(cudaGetLastError(), "batch finish launch");
 }
@@ -1069,9 +1191,11 @@ int launchGatherEval(const GatherEvalArgs& a, cudaStream_t s)
 
 int launchLbfgs(const LbfgsArgs& a, cudaStream_t s)
 {
-	const int threads = 256;
-	const int blocks = (int)((a.Q * 32ull + threads - 1) / threads);
-	lbfgsKernel<<<std::max(blocks, 1), threads, 0, s>>>(a);
+	// up to 128 parameters (every packed layout, and general ones that small) fit in registers
+	if (a.Q > 0 && a.P <= 128)
+		lbfgsKernel<4><<<a.Q, 32, 0, s>>>(a);
+	else if (a.Q > 0)
+		lbfgsKernel<0><<<a.Q, 32, 0, s>>>(a);
 	countLaunches(1);
 	return cudaCheck(cudaGetLastError(), "L-BFGS launch");
 }
