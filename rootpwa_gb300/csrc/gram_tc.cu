@@ -801,41 +801,64 @@ __global__ void __launch_bounds__(kThreadsHL, 1) gramTcHiLoKernel(const __grid_c
 
 // FP64 sum of the CTAs' partials; assembles the Hermitian matrix (upper
 // triangle from Re and D, lower mirrored, real diagonal).  sym: the first
-// partial is S with Re = (S + S^T) / 2 (the hi/lo kernel).  One warp per
-// element: lane l sums CTAs l, l + 32, ... in order, a fixed butterfly
-// combines the lanes (the same order on every run).
-__global__ void __launch_bounds__(256) gramTcReduceKernel(const float* partials, int grid, int W, int N, int sym,
-                                                          double* out)
+// partial is S with Re = (S + S^T) / 2 (the hi/lo kernel).  Order of the sum,
+// the same on every run: 32 sub-sums over CTAs l, l + 32, ..., combined
+// pairwise at distances 16, 8, 4, 2, 1.  A block takes 32 elements of the upper
+// triangle (146 blocks for 96 columns), a thread four of the sub-sums of one
+// element.  What bounds it is the FP64 pipe (eight operations per element and
+// CTA, conversions included: 10 us of its rate for 96 columns); one warp per
+// element spent as much again on the butterfly and waited for one CTA's loads
+// at a time: 28 us, 19 now.
+constexpr int kRedSub = 8;  // threads per element
+__global__ void __launch_bounds__(32 * kRedSub) gramTcReduceKernel(const float* __restrict__ partials, int grid, int W,
+                                                                   int N, int sym, double* out)
 {
-	const int lane = threadIdx.x & 31;
-	const int nWarps = (int)((gridDim.x * blockDim.x) >> 5);
-	const int n = W * W;
-	for (int e = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); e < n; e += nWarps) {
-		const int i = e / W, j = e - i * W;
-		if (i > j)
-			continue;
-		double re = 0., im = 0.;
-		for (int c = lane; c < grid; c += 32) {
-			const float* Re = partials + (size_t)c * 2 * 128 * N;
-			const float* D = Re + (size_t)128 * N;
-			re += sym ? 0.5 * ((double)Re[(size_t)i * N + j] + (double)Re[(size_t)j * N + i])
-			          : (double)Re[(size_t)i * N + j];
-			im += (double)D[(size_t)i * N + j] - (double)D[(size_t)j * N + i];
+	__shared__ double sRe[kRedSub][32], sIm[kRedSub][32];
+	const int lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
+	int i = 0, j = (int)blockIdx.x * 32 + lane;
+	const bool use = j < W * (W + 1) / 2;
+	if (use) {
+		while (j >= W - i) {
+			j -= W - i;
+			++i;
 		}
+		j += i;
+		double re[4] = {0., 0., 0., 0.}, im[4] = {0., 0., 0., 0.};
+		const size_t step = (size_t)2 * 128 * N, toD = (size_t)128 * N;
+		const float* pij = partials + (size_t)i * N + j;
+		const float* pji = partials + (size_t)j * N + i;
+		for (int c0 = sub; c0 < grid; c0 += 32) {
+			float v[4][4];
 #pragma unroll
-		for (int o = 16; o > 0; o >>= 1) {
-			re += __shfl_xor_sync(0xffffffffu, re, o);
-			im += __shfl_xor_sync(0xffffffffu, im, o);
+			for (int m = 0; m < 4; ++m) {
+				const size_t o = (size_t)min(c0 + 8 * m, grid - 1) * step;
+				v[m][0] = __ldg(pij + o);
+				v[m][1] = __ldg(pji + o);
+				v[m][2] = __ldg(pij + o + toD);
+				v[m][3] = __ldg(pji + o + toD);
+			}
+#pragma unroll
+			for (int m = 0; m < 4; ++m)
+				if (c0 + 8 * m < grid) {
+					re[m] += sym ? 0.5 * ((double)v[m][0] + (double)v[m][1]) : (double)v[m][0];
+					im[m] += (double)v[m][2] - (double)v[m][3];
+				}
 		}
-		if (lane == 0) {
-			if (i == j)
-				im = 0.;
-			out[(size_t)e * 2] = re;
-			out[(size_t)e * 2 + 1] = im;
-			out[((size_t)j * W + i) * 2] = re;
-			out[((size_t)j * W + i) * 2 + 1] = -im;
-		}
+		sRe[sub][lane] = (re[0] + re[2]) + (re[1] + re[3]);
+		sIm[sub][lane] = (im[0] + im[2]) + (im[1] + im[3]);
 	}
+	__syncthreads();
+	if (!use || sub > 0)
+		return;
+	auto tree = [&](const double(*v)[32]) {
+		return ((v[0][lane] + v[4][lane]) + (v[2][lane] + v[6][lane])) +
+		       ((v[1][lane] + v[5][lane]) + (v[3][lane] + v[7][lane]));
+	};
+	const double re = tree(sRe), im = i == j ? 0. : tree(sIm);
+	out[((size_t)i * W + j) * 2] = re;
+	out[((size_t)i * W + j) * 2 + 1] = im;
+	out[((size_t)j * W + i) * 2] = re;
+	out[((size_t)j * W + i) * 2 + 1] = -im;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -963,9 +986,8 @@ int launchGramTc(const GramArgs& g, int precision, int numSMs, cudaStream_t s, d
 	}
 	countLaunches(1);
 	PWA_CHECK_RET(cudaCheck(cudaGetLastError(), "gram TC launch"));
-	const int n = g.W * g.W;
-	const int blocks = std::max(1, std::min(4096, (n + 7) / 8));  // eight warps per block, one per element
-	gramTcReduceKernel<<<blocks, 256, 0, s>>>(a.partials, grid, g.W, a.N, hiLo ? 1 : 0, out);
+	gramTcReduceKernel<<<(g.W * (g.W + 1) / 2 + 31) / 32, 32 * kRedSub, 0, s>>>(a.partials, grid, g.W, a.N, hiLo ? 1 : 0,
+	                                                                            out);
 	countLaunches(1);
 	return cudaCheck(cudaGetLastError(), "gram TC reduce launch");
 }

@@ -1335,8 +1335,11 @@ int pwa_likelihood_hessian(pwa_likelihood* L, const double* par, double* H)
 		PWA_TRY(cudaCheck(cudaMemsetAsync(dY2.as<float2>() + (size_t)nY2 * slab, 0,
 		                                  (size_t)(rows2 - nY2) * slab * sizeof(float2), s),
 		                  "memset"));
-	// dG (n x n) += the weighted Gram of the n rows of Y over K events
-	auto gramAdd = [&](const float2* Y, uint32_t n, uint32_t G, uint32_t ng, const double* w, uint64_t K,
+	// dG (n x n) += the weighted Gram of the n rows of Y over K events: the
+	// blocks with one of the first `need` rows, and the last row's norm (of the
+	// first set the conj(d) x conj(d) blocks are not used: 6 of 28 pairs of
+	// groups for 2 x 87 slots)
+	auto gramAdd = [&](const float2* Y, uint32_t n, uint32_t need, uint32_t G, uint32_t ng, const double* w, uint64_t K,
 	                   double* dG) -> int {
 		GramArgs g{};
 		g.K = K;
@@ -1349,7 +1352,8 @@ int pwa_likelihood_hessian(pwa_likelihood* L, const double* par, double* H)
 			PWA_TRY(launchGramTc(g, PWA_PRECISION_TF32X3, L->numSMs, s, dBlk.as<double>(), dPart.as<double>(), scratch));
 			return launchGramBlockAdd(dBlk.as<double>(), (int)n, (int)n, 0, 0, (int)n, 1, 1, dG, s);
 		}
-		for (uint32_t ga = 0; ga < ng; ++ga)
+		const uint32_t nga = std::min(ng - 1, (need + G - 1) / G);
+		for (uint32_t ga = 0; ga < nga; ++ga)
 			for (uint32_t gb = ga + 1; gb < ng; ++gb) {
 				g.amps = Y + (size_t)ga * G * slab;
 				g.W = (int)(2 * G);
@@ -1357,9 +1361,9 @@ int pwa_likelihood_hessian(pwa_likelihood* L, const double* par, double* H)
 				PWA_TRY(launchGramTc(g, PWA_PRECISION_TF32X3, L->numSMs, s, dBlk.as<double>(), dPart.as<double>(),
 				                     scratch));
 				// group ga's diagonal block from its pair with ga + 1, the last
-				// group's from the last pair
+				// group's from its last pair
 				PWA_TRY(launchGramBlockAdd(dBlk.as<double>(), (int)(2 * G), (int)G, (int)ga, (int)gb, (int)n,
-				                           gb == ga + 1 ? 1 : 0, (ga + 2 == ng && gb + 1 == ng) ? 1 : 0, dG, s));
+				                           gb == ga + 1 ? 1 : 0, (ga + 1 == nga && gb + 1 == ng) ? 1 : 0, dG, s));
 			}
 		return kOk;
 	};
@@ -1368,8 +1372,8 @@ int pwa_likelihood_hessian(pwa_likelihood* L, const double* par, double* H)
 		PWA_TRY(launchHessPrep(L->amps.as<float2>(), L->nEvents, L->storeB, e0, slab, (int)L->nW[0], (int)W, (int)R,
 		                       (int)P, dHP.as<double>(), L->dSlotRe.as<int>(), L->dSlotIm.as<int>(), dY1.as<float2>(),
 		                       dY2.as<float2>(), dW1.as<double>(), dW2.as<double>(), s));
-		PWA_TRY(gramAdd(dY1.as<float2>(), nY1, gs1, ng1, dW1.as<double>(), K, dG1.as<double>()));
-		PWA_TRY(gramAdd(dY2.as<float2>(), nY2, gs2, ng2, dW2.as<double>(), K, dG2.as<double>()));
+		PWA_TRY(gramAdd(dY1.as<float2>(), nY1, nS, gs1, ng1, dW1.as<double>(), K, dG1.as<double>()));
+		PWA_TRY(gramAdd(dY2.as<float2>(), nY2, nY2, gs2, ng2, dW2.as<double>(), K, dG2.as<double>()));
 	}
 	unsigned gramErr = 0;
 	PWA_TRY(cudaCheck(cudaMemcpyAsync(&gramErr, dErrG.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "D2H flag"));
