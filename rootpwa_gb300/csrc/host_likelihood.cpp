@@ -358,6 +358,17 @@ int autotunePlan(pwa_likelihood* L, const std::vector<FdfPlan>& cands)
 	return kOk;
 }
 
+// a part of a larger device allocation
+struct DevPart {
+	void* p;
+	size_t bytes;
+	template <class T>
+	T* as() const
+	{
+		return static_cast<T*>(p);
+	}
+};
+
 }  // namespace
 
 extern "C" {
@@ -1312,17 +1323,25 @@ int pwa_likelihood_hessian(pwa_likelihood* L, const double* par, double* H)
 	slab = std::max<uint64_t>(1024, std::min<uint64_t>(slab, (L->nEvents + 63) / 64 * 64)) / 64 * 64;
 	const uint32_t maxGram = std::max(ng1 > 1 ? 2 * gs1 : gs1, ng2 > 1 ? 2 * gs2 : gs2);
 	const size_t scratch = gramTcScratchFloats((int)maxGram, L->numSMs) / 2 + 1;
-	DevBuf dY1, dY2, dW1, dW2, dPart, dBlk, dErrG, dG1, dG2, dHP;
-	PWA_TRY(dY1.alloc((size_t)rows1 * slab * sizeof(float2), "hessian operand"));
-	PWA_TRY(dY2.alloc((size_t)rows2 * slab * sizeof(float2), "hessian operand"));
-	PWA_TRY(dW1.alloc(slab * sizeof(double), "hessian weights"));
-	PWA_TRY(dW2.alloc(slab * sizeof(double), "hessian weights"));
-	PWA_TRY(dPart.alloc(scratch * sizeof(double), "hessian gram partials"));
-	PWA_TRY(dBlk.alloc((size_t)maxGram * maxGram * 2 * sizeof(double), "hessian gram block"));
-	PWA_TRY(dErrG.alloc(sizeof(unsigned), "flag"));
-	PWA_TRY(dG1.alloc((size_t)nY1 * nY1 * 2 * sizeof(double), "hessian gram"));
-	PWA_TRY(dG2.alloc((size_t)nY2 * nY2 * 2 * sizeof(double), "hessian gram"));
-	PWA_TRY(dHP.alloc(P * sizeof(double), "hessian parameters"));
+	// one device allocation for all of it, in 256-byte aligned parts: with one
+	// for each of ten buffers allocating and freeing took 1.0 ms more than with
+	// one; a call for 87 waves, rank 2 and 250,001 events took 4.73 ms, now 4.34
+	DevPart dY1{nullptr, (size_t)rows1 * slab * sizeof(float2)}, dY2{nullptr, (size_t)rows2 * slab * sizeof(float2)},
+	    dW1{nullptr, slab * sizeof(double)}, dW2{nullptr, slab * sizeof(double)}, dPart{nullptr, scratch * sizeof(double)},
+	    dBlk{nullptr, (size_t)maxGram * maxGram * 2 * sizeof(double)}, dErrG{nullptr, sizeof(unsigned)},
+	    dG1{nullptr, (size_t)nY1 * nY1 * 2 * sizeof(double)}, dG2{nullptr, (size_t)nY2 * nY2 * 2 * sizeof(double)},
+	    dHP{nullptr, P * sizeof(double)};
+	DevPart* const parts[] = {&dY1, &dY2, &dW1, &dW2, &dPart, &dBlk, &dErrG, &dG1, &dG2, &dHP};
+	size_t total = 0;
+	for (const DevPart* q : parts)
+		total += (q->bytes + 255) / 256 * 256;
+	DevBuf arena;
+	PWA_TRY(arena.alloc(total, "hessian workspace"));
+	total = 0;
+	for (DevPart* q : parts) {
+		q->p = arena.as<unsigned char>() + total;
+		total += (q->bytes + 255) / 256 * 256;
+	}
 	PWA_TRY(cudaCheck(cudaMemcpyAsync(dHP.p, par, P * sizeof(double), cudaMemcpyHostToDevice, s), "H2D par"));
 	PWA_TRY(cudaCheck(cudaMemsetAsync(dG1.p, 0, dG1.bytes, s), "memset"));
 	PWA_TRY(cudaCheck(cudaMemsetAsync(dG2.p, 0, dG2.bytes, s), "memset"));
