@@ -194,5 +194,46 @@ __device__ __forceinline__ void fdfTail(const FdfArgs& a, unsigned* sLast, doubl
 	}
 }
 
+// Placement of the phase-1 roles in a warp.  Roles are numbered as if lane
+// bits 0.. were the wave slice and the bits above the event; role bit i is bit
+// bit(i) of the lane.  A 16-byte load of V, the same for all events of a wave
+// slice, takes two passes of the shared-memory pipe when each lane has its
+// address in common with lane ^ 1 or lane ^ 2 and four otherwise, so an event
+// bit goes to lane bit 0; the lanes of a quarter (one-event variant: half) of
+// a warp still cover distinct banks with their amplitude loads, as wave
+// slices' rows are rotated against each other.  With the slice in the low lane
+// bits, per FdF: 64 waves of rank 4, 1 M events 195 us, now 179; 87 waves of
+// rank 2 144, now 142; 45 waves of rank 3 125, now 118.
+template <int E, int NE>
+struct LaneRoles {
+	__host__ __device__ static constexpr int bit(int i)
+	{
+		return E == 128  ? (i == 0 ? 1 : i == 1 ? 2 : i == 2 ? 0 : i)
+		       : E == 64 ? (NE == 1 ? (i == 3 ? 0 : i < 3 ? i + 1 : i) : (i == 0 ? 3 : i == 3 ? 0 : i))
+		                 : (i == 0 ? 4 : i == 4 ? 0 : i);
+	}
+	__device__ static __forceinline__ int role(int lane)
+	{
+		int r = 0;
+#pragma unroll
+		for (int i = 0; i < 5; ++i)
+			r |= ((lane >> bit(i)) & 1) << i;
+		return r;
+	}
+	__device__ static __forceinline__ int lane(int role)
+	{
+		int l = 0;
+#pragma unroll
+		for (int i = 0; i < 5; ++i)
+			l |= ((role >> i) & 1) << bit(i);
+		return l;
+	}
+	// lane distance of the role distance o (a power of two)
+	__host__ __device__ static constexpr int dist(int o)
+	{
+		return o == 1 ? 1 << bit(0) : o == 2 ? 1 << bit(1) : o == 4 ? 1 << bit(2) : o == 8 ? 1 << bit(3) : 1 << bit(4);
+	}
+};
+
 }  // namespace
 }  // namespace pwa

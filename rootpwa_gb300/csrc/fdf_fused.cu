@@ -12,7 +12,7 @@
 //     amplitudes (a quarter-warp holds two event pairs x four slices with
 //     distinct store rotations, so its loads hit all 32 banks once);
 //   * the coherent sums S of the pair are combined over the 8 lanes of the
-//     pair (a reduce-scatter over lane bit 16, a butterfly over bits 0-1);
+//     pair (a reduce-scatter over role bit 4, a butterfly over bits 0-1);
 //     each lane then has L, c and c S of one event and gets the other
 //     event's c S with one shuffle;
 //   * the lane reads the same amplitudes again (its waves, its two events)
@@ -140,11 +140,13 @@ __global__ void __launch_bounds__(kThreads, 1) fdfFusedKernel(const FdfArgs a, c
 	// lane roles: event pair pm2 of the warp (events pe0, pe0 + 1), wave
 	// slice ph2 (waves w = ph2 mod 8 of each reflectivity); after the
 	// combination the lane holds event pe0 + mine
-	const int phLo = lane & 3;
-	const int pm2 = ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-	const int ph2 = phLo + 4 * (lane >> 4);
+	using Roles = LaneRoles<E, 2>;
+	const int role = Roles::role(lane);
+	const int phLo = role & 3;
+	const int pm2 = ((role >> 3) & 1) * 2 + ((role >> 2) & 1);
+	const int ph2 = phLo + 4 * (role >> 4);
 	const int pe0 = warp * EPW + 2 * pm2;
-	const int mine = (lane >> 4) & 1;
+	const int mine = (role >> 4) & 1;
 	const int n0 = ph2 < W0 ? (W0 - 1 - ph2) / 8 + 1 : 0;
 	const int wS1 = W0 + (((ph2 - W0) % 8) + 8) % 8;
 	const int n1 = wS1 < W ? (W - 1 - wS1) / 8 + 1 : 0;
@@ -269,12 +271,12 @@ __global__ void __launch_bounds__(kThreads, 1) fdfFusedKernel(const FdfArgs a, c
 				const float2 (&Se)[R][2] = e ? S1 : S0;
 				float2 keep = mine ? Se[r][1] : Se[r][0];
 				const float2 send = mine ? Se[r][0] : Se[r][1];
-				keep.x += __shfl_xor_sync(0xffffffffu, send.x, 16);
-				keep.y += __shfl_xor_sync(0xffffffffu, send.y, 16);
+				keep.x += __shfl_xor_sync(0xffffffffu, send.x, Roles::dist(16));
+				keep.y += __shfl_xor_sync(0xffffffffu, send.y, Roles::dist(16));
 #pragma unroll
 				for (int o = 1; o < 4; o <<= 1) {
-					keep.x += __shfl_xor_sync(0xffffffffu, keep.x, o);
-					keep.y += __shfl_xor_sync(0xffffffffu, keep.y, o);
+					keep.x += __shfl_xor_sync(0xffffffffu, keep.x, Roles::dist(o));
+					keep.y += __shfl_xor_sync(0xffffffffu, keep.y, Roles::dist(o));
 				}
 				S[r][e] = keep;
 			}
@@ -300,8 +302,8 @@ __global__ void __launch_bounds__(kThreads, 1) fdfFusedKernel(const FdfArgs a, c
 #pragma unroll
 				for (int e = 0; e < 2; ++e) {
 					const float2 t = make_float2(c * S[r][e].x, c * S[r][e].y);
-					const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, t.x, 16),
-					                             __shfl_xor_sync(0xffffffffu, t.y, 16));
+					const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, t.x, Roles::dist(16)),
+					                             __shfl_xor_sync(0xffffffffu, t.y, Roles::dist(16)));
 					T0[e][r] = mine ? o : t;
 					T1[e][r] = mine ? t : o;
 				}
@@ -337,7 +339,10 @@ __global__ void __launch_bounds__(kThreads, 1) fdfFusedKernel(const FdfArgs a, c
 
 		// fold the FP32 partials every kFoldF tiles and after the last tile
 		if ((k + 1) % kFoldF == 0 || k + 1 == myTiles) {
-			const float ll = warpSum(llPart), cs = warpSum(cPart);
+			// (summed in the order of the roles)
+			const int from = Roles::lane(lane);
+			const float ll = warpSum(__shfl_sync(0xffffffffu, llPart, from));
+			const float cs = warpSum(__shfl_sync(0xffffffffu, cPart, from));
 			llPart = 0.f;
 			cPart = 0.f;
 			if (lane == 0) {
@@ -350,7 +355,7 @@ __global__ void __launch_bounds__(kThreads, 1) fdfFusedKernel(const FdfArgs a, c
 				}
 			}
 			if (a.withGrad) {
-				// the four lanes of a wave slice (lane bits 2 and 3) hold the
+				// the four lanes of a wave slice (role bits 2 and 3) hold the
 				// same waves for different event pairs; the shuffles run on
 				// all lanes, the shared-memory adds on the first lane of each
 				// slice only
@@ -360,10 +365,10 @@ __global__ void __launch_bounds__(kThreads, 1) fdfFusedKernel(const FdfArgs a, c
 #pragma unroll
 					for (int r = 0; r < R; ++r) {
 						float gx = Gn[j][r].x, gy = Gn[j][r].y;
-						gx += __shfl_xor_sync(0xffffffffu, gx, 4);
-						gy += __shfl_xor_sync(0xffffffffu, gy, 4);
-						gx += __shfl_xor_sync(0xffffffffu, gx, 8);
-						gy += __shfl_xor_sync(0xffffffffu, gy, 8);
+						gx += __shfl_xor_sync(0xffffffffu, gx, Roles::dist(4));
+						gy += __shfl_xor_sync(0xffffffffu, gy, Roles::dist(4));
+						gx += __shfl_xor_sync(0xffffffffu, gx, Roles::dist(8));
+						gy += __shfl_xor_sync(0xffffffffu, gy, Roles::dist(8));
 						if (NEG > 0 && pm2 == 0 && j < n0 &&
 						    smemInBounds(smemAddr(Gw + (r * W + ph2 + 8 * j) * 2), 16u, smemAddr(Gw), smemAddr(Gw + nG),
 						                 a.devErr)) {
@@ -378,10 +383,10 @@ __global__ void __launch_bounds__(kThreads, 1) fdfFusedKernel(const FdfArgs a, c
 #pragma unroll
 					for (int r = 0; r < R; ++r) {
 						float gx = Gp[j][r].x, gy = Gp[j][r].y;
-						gx += __shfl_xor_sync(0xffffffffu, gx, 4);
-						gy += __shfl_xor_sync(0xffffffffu, gy, 4);
-						gx += __shfl_xor_sync(0xffffffffu, gx, 8);
-						gy += __shfl_xor_sync(0xffffffffu, gy, 8);
+						gx += __shfl_xor_sync(0xffffffffu, gx, Roles::dist(4));
+						gy += __shfl_xor_sync(0xffffffffu, gy, Roles::dist(4));
+						gx += __shfl_xor_sync(0xffffffffu, gx, Roles::dist(8));
+						gy += __shfl_xor_sync(0xffffffffu, gy, Roles::dist(8));
 						if (POS > 0 && pm2 == 0 && j < n1 &&
 						    smemInBounds(smemAddr(Gw + (r * W + wS1 + 8 * j) * 2), 16u, smemAddr(Gw), smemAddr(Gw + nG),
 						                 a.devErr)) {

@@ -179,7 +179,9 @@ __global__ void __launch_bounds__(kThreads, 1) fdfMainKernel(const FdfArgs a, co
 	__syncthreads();
 
 	// phase-1 role: event pe of the tile, wave slice ph (waves w = ph mod H)
-	const int pm = lane / H, ph = lane - pm * H;
+	using Roles = LaneRoles<E, NE>;
+	const int role = Roles::role(lane);
+	const int pm = role / H, ph = role - pm * H;
 	const int pe = warp * EPW + pm;
 	const int wStart1 = W0 + (((ph - W0) % H) + H) % H;  // first positive-reflectivity wave of this slice
 	// phase-2 role: the warp owns waves [wBase, wBase + nWarpWaves) of reflectivity wRefl
@@ -309,8 +311,8 @@ __global__ void __launch_bounds__(kThreads, 1) fdfMainKernel(const FdfArgs a, co
 						S[r][e] = Sa[r][e];
 #pragma unroll
 						for (int o = 1; o < H; o <<= 1) {
-							S[r][e].x += __shfl_xor_sync(0xffffffffu, S[r][e].x, o);
-							S[r][e].y += __shfl_xor_sync(0xffffffffu, S[r][e].y, o);
+							S[r][e].x += __shfl_xor_sync(0xffffffffu, S[r][e].x, Roles::dist(o));
+							S[r][e].y += __shfl_xor_sync(0xffffffffu, S[r][e].y, Roles::dist(o));
 						}
 					}
 				pe1 = pe;
@@ -323,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, 1) fdfMainKernel(const FdfArgs a, co
 				// (2 quads x 4 slices with distinct store rotations) covers
 				// all 32 banks once in both loads.
 				static_assert(E == 128, "four events per lane need 128-event tiles");
-				const int kLo = lane & 3, quad = (lane >> 2) & 1, sHi = (lane >> 3) & 3;
+				const int kLo = role & 3, quad = (role >> 2) & 1, sHi = (role >> 3) & 3;
 				const int ph4 = kLo + 4 * sHi;          // wave slice: waves w = ph4 mod 16
 				const int pe0 = warp * EPW + 4 * quad;  // the quad's first event
 				const int rot1 = (int)storeRot((uint32_t)ph4, (uint32_t)E);
@@ -362,10 +364,10 @@ __global__ void __launch_bounds__(kThreads, 1) fdfMainKernel(const FdfArgs a, co
 #pragma unroll 1
 				for (int w = wS1; w < W; w += 16)
 					mac4(w, SP);
-				// reduce-scatter over lane bit 16 (slot) and bit 8 (event of
+				// reduce-scatter over role bit 4 (slot) and bit 3 (event of
 				// the slot), butterfly over bits 0-1: the lane ends with the
 				// sums of event pe0 + 2 (bs ^ quad) + be
-				const int bs = (lane >> 4) & 1, be = (lane >> 3) & 1;
+				const int bs = (role >> 4) & 1, be = (role >> 3) & 1;
 #pragma unroll
 				for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -375,18 +377,18 @@ __global__ void __launch_bounds__(kThreads, 1) fdfMainKernel(const FdfArgs a, co
 						float2 k1 = bs ? Se[1][1][r] : Se[0][1][r];
 						const float2 s0 = bs ? Se[0][0][r] : Se[1][0][r];
 						const float2 s1 = bs ? Se[0][1][r] : Se[1][1][r];
-						k0.x += __shfl_xor_sync(0xffffffffu, s0.x, 16);
-						k0.y += __shfl_xor_sync(0xffffffffu, s0.y, 16);
-						k1.x += __shfl_xor_sync(0xffffffffu, s1.x, 16);
-						k1.y += __shfl_xor_sync(0xffffffffu, s1.y, 16);
+						k0.x += __shfl_xor_sync(0xffffffffu, s0.x, Roles::dist(16));
+						k0.y += __shfl_xor_sync(0xffffffffu, s0.y, Roles::dist(16));
+						k1.x += __shfl_xor_sync(0xffffffffu, s1.x, Roles::dist(16));
+						k1.y += __shfl_xor_sync(0xffffffffu, s1.y, Roles::dist(16));
 						float2 keep = be ? k1 : k0;
 						const float2 send = be ? k0 : k1;
-						keep.x += __shfl_xor_sync(0xffffffffu, send.x, 8);
-						keep.y += __shfl_xor_sync(0xffffffffu, send.y, 8);
+						keep.x += __shfl_xor_sync(0xffffffffu, send.x, Roles::dist(8));
+						keep.y += __shfl_xor_sync(0xffffffffu, send.y, Roles::dist(8));
 #pragma unroll
 						for (int o = 1; o < 4; o <<= 1) {
-							keep.x += __shfl_xor_sync(0xffffffffu, keep.x, o);
-							keep.y += __shfl_xor_sync(0xffffffffu, keep.y, o);
+							keep.x += __shfl_xor_sync(0xffffffffu, keep.x, Roles::dist(o));
+							keep.y += __shfl_xor_sync(0xffffffffu, keep.y, Roles::dist(o));
 						}
 						S[r][e] = keep;
 					}
@@ -403,9 +405,9 @@ __global__ void __launch_bounds__(kThreads, 1) fdfMainKernel(const FdfArgs a, co
 				constexpr int PQ = E / 64;    // pairs per quarter-warp
 				constexpr int QPH = 8 / PQ;   // wave slices per quarter-warp
 				static_assert(PQ * QPH == 8 && 2 * PQ == PPW && 2 * QPH == H2, "two-event phase-1 shape");
-				const int phLo = lane & (QPH - 1);
-				const int pm2 = ((lane >> 3) & 1) * PQ + ((lane / QPH) & (PQ - 1));
-				const int ph2 = phLo + QPH * (lane >> 4);
+				const int phLo = role & (QPH - 1);
+				const int pm2 = ((role >> 3) & 1) * PQ + ((role / QPH) & (PQ - 1));
+				const int ph2 = phLo + QPH * (role >> 4);
 				const int pe0 = warp * EPW + 2 * pm2;
 				// H2 is a multiple of 512 / E: one rotation for all rows of the slice
 				const int rot1 = (int)storeRot((uint32_t)ph2, (uint32_t)E);
@@ -440,7 +442,7 @@ __global__ void __launch_bounds__(kThreads, 1) fdfMainKernel(const FdfArgs a, co
 				// a reduce-scatter over the slice bit 16 (lanes with that bit
 				// keep the second event) and a butterfly over the remaining
 				// slice bits
-				const int mine = (lane >> 4) & 1;
+				const int mine = (role >> 4) & 1;
 #pragma unroll
 				for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -448,12 +450,12 @@ __global__ void __launch_bounds__(kThreads, 1) fdfMainKernel(const FdfArgs a, co
 						const float2 (&Se)[R][2] = e ? S1 : S0;
 						float2 keep = mine ? Se[r][1] : Se[r][0];
 						const float2 send = mine ? Se[r][0] : Se[r][1];
-						keep.x += __shfl_xor_sync(0xffffffffu, send.x, 16);
-						keep.y += __shfl_xor_sync(0xffffffffu, send.y, 16);
+						keep.x += __shfl_xor_sync(0xffffffffu, send.x, Roles::dist(16));
+						keep.y += __shfl_xor_sync(0xffffffffu, send.y, Roles::dist(16));
 #pragma unroll
 						for (int o = 1; o < QPH; o <<= 1) {
-							keep.x += __shfl_xor_sync(0xffffffffu, keep.x, o);
-							keep.y += __shfl_xor_sync(0xffffffffu, keep.y, o);
+							keep.x += __shfl_xor_sync(0xffffffffu, keep.x, Roles::dist(o));
+							keep.y += __shfl_xor_sync(0xffffffffu, keep.y, Roles::dist(o));
 						}
 						S[r][e] = keep;
 					}
@@ -552,7 +554,10 @@ __global__ void __launch_bounds__(kThreads, 1) fdfMainKernel(const FdfArgs a, co
 		// fold the FP32 tile partials every foldTiles(reduction) tiles and after the last tile
 		if (--foldLeft == 0 || k + 1 == myTiles) {
 			foldLeft = foldTiles(a.reduction);
-			const float ll = warpSum(llPart), cs = warpSum(cPart);
+			// (summed in the order of the roles)
+			const int from = Roles::lane(lane);
+			const float ll = warpSum(__shfl_sync(0xffffffffu, llPart, from));
+			const float cs = warpSum(__shfl_sync(0xffffffffu, cPart, from));
 			llPart = 0.f;
 			cPart = 0.f;
 			if (lane == 0) {
