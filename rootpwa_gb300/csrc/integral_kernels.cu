@@ -415,7 +415,8 @@ struct TriArgs {
 // One block: `slices` chunks of K, one thread tile per thread.  KT steps of
 // K are staged per round in two buffers: the FP32 operands by asynchronous
 // copies that run while the previous round is used (held in registers for
-// that time, they spilled: 250 against 130 us at 50 waves), the FP64 ones
+// that time, they spilled: 355 against 247 us per weighted call of 50 waves,
+// 300,001 events), the FP64 ones
 // converted and weighted on the way, beside which the FP64 pipe hides their
 // loads.
 template <typename Acc, typename In, int KT, bool WT>
