@@ -1270,9 +1270,8 @@ def run_isobar(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "traffic": None, "peak_kind": peak_kind,
                      "note": ("algorithmic bytes (96 B in + 8 B per wave out per event, complex64 mode); the "
-                              "kernel is not HBM-bound: it is latency-bound on the per-wave FP32 arithmetic "
-                              "and its plan loads (ncu: issue active 49 %, DRAM < 1 %; "
-                              "profiles/isobar_amplitude_kernel_3pi88.md)")},
+                              "kernel is not HBM-bound: it is latency-bound at 16 warps per SM (ncu: SM "
+                              "throughput 41 %, DRAM 2 %; profiles/kernels_of_the_measured_workloads.md)")},
         "cpu_baseline": {"value": n_check / t_cpu, "unit": "events/s", "cores": 1, "kind": "port",
                          "sample": "FP64 oracle (numpy) on %d events x %d waves" % (n_check, W)},
         "max_rel_err_vs_oracle": err,
