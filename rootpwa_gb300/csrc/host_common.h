@@ -140,12 +140,12 @@ using namespace pwa;
 // ampIntegralMatrix: raw sums and the wave list
 // ===========================================================================
 // device buffers and stream of integrate(), kept by an integral between
-// calls on one device (the output matrix, the error flag, the Gram partials,
-// the rows' range and the event weights: no allocation per call once they have their size)
+// calls on one device (the output matrix, the error flag, the Gram partials
+// and the event weights: no allocation per call once they have their size)
 struct GramScratch {
 	int dev = -1;
 	cudaStream_t stream = nullptr;
-	DevBuf out, err, part, rowMax, weights, rawWeights;
+	DevBuf out, err, part, weights, rawWeights;
 	GramScratch() = default;
 	GramScratch(const GramScratch&) = delete;
 	GramScratch& operator=(const GramScratch&) = delete;
@@ -155,7 +155,6 @@ struct GramScratch {
 		out.release();
 		err.release();
 		part.release();
-		rowMax.release();
 		weights.release();
 		rawWeights.release();
 		if (stream)

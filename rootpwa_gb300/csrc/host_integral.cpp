@@ -12,12 +12,12 @@
 namespace {
 
 // Sums the GPU Gram kernel for integrate().  Event weights come either
-// expanded (weightK; weights01: all 0 or 1) or as the caller's weight stream
-// with one entry per event (rawWeights: 1 / w per sub-amplitude and the sum of
-// 1 / w, *weightSum, are formed on the device).
+// expanded (weightK) or as the caller's weight stream with one entry per event
+// (rawWeights: 1 / w per sub-amplitude and the sum of 1 / w, *weightSum, are
+// formed on the device).
 int gramOnDevice(GramScratch& sc, uint32_t W, const void* amps, uint64_t nEvents, uint32_t nSub, int ampType,
-                 int memory, const std::vector<double>& weightK, const double* rawWeights, bool weights01, uint64_t K,
-                 int precision, std::vector<cplx>& out, double* weightSum)
+                 int memory, const std::vector<double>& weightK, const double* rawWeights, uint64_t K, int precision,
+                 std::vector<cplx>& out, double* weightSum)
 {
 	int dev, sms;
 	size_t smem;
@@ -142,11 +142,6 @@ int gramOnDevice(GramScratch& sc, uint32_t W, const void* amps, uint64_t nEvents
 		const int chunks = gramSimtChunks(g, precision, sms);
 		g.chunks = chunks;
 		PWA_TRY(dPart.ensure((size_t)chunks * W * W * 2 * sizeof(double), "gram partials"));
-		if (precision == PWA_PRECISION_FP64) {
-			PWA_TRY(sc.rowMax.ensure((1 + (size_t)chunks * W) * sizeof(unsigned), "row range"));
-			g.rowMax = sc.rowMax.as<unsigned>();
-		}
-		g.weights01 = weights01;
 		g.partials = dPart.as<double>();
 		PWA_TRY(launchGramSimt(g, precision, s));
 		PWA_TRY(launchGramReduce(g.partials, chunks, (int)W, dOut.as<double>(), 0, s));
@@ -300,7 +295,7 @@ int pwa_integral_integrate(pwa_integral* I, uint32_t nWaves, const char* const* 
 			return setError(kErrOom, "out of host memory");
 		double devSum = 0.;
 		PWA_TRY(gramOnDevice(*I->scratch.p, nWaves, amps, nEvents, nSubAmps, ampType, memory, weightK,
-		                     rawWeights ? weights : nullptr, !useWeight, K, precision, result, &devSum));
+		                     rawWeights ? weights : nullptr, K, precision, result, &devSum));
 		if (rawWeights)
 			wsum = devSum;
 	} else {

@@ -4,12 +4,12 @@
 // (decayAmplitude/ampIntegralMatrix.cc:408-469)
 //   I_ij = sum_k w_k A_{i,k} conj(A_{j,k})
 // over K = events x sub-amplitudes.  gramTriKernel forms the upper triangle
-// in thread tiles of 4 rows (FP32, FP64, or FP64 accuracy from FP32
-// arithmetic) for one contiguous chunk of K per thread group; chunk partials are
-// summed in FP64 by a second kernel, which also mirrors the upper triangle
-// into the lower one (the reference's matrix is exactly Hermitian, since
-// a conj(b) and b conj(a) round identically).  Wave sets too wide for its
-// shared memory take gramSimtKernel (64 x 64 output tiles).
+// in 4 x 4 thread tiles (FP32 or FP64 products and sums) for one contiguous
+// chunk of K per thread group; chunk partials are summed in FP64 by a second
+// kernel, which also mirrors the upper triangle into the lower one (the
+// reference's matrix is exactly Hermitian, since a conj(b) and b conj(a) round
+// identically).  Wave sets too wide for its shared memory take gramSimtKernel
+// (64 x 64 output tiles).
 // The tensor-core variant lives in gram_tc.cu.
 
 #include "pwa_internal.h"
@@ -134,54 +134,15 @@ __global__ void __launch_bounds__(256) gramSimtKernel(const In* __restrict__ amp
 // Small wave sets put several chunks of K side by side in one block.
 //
 // What bounds it: the arithmetic pipes.  GB300 issues 2 FP64 FMAs per clock
-// and SM against 128 FP32 ones, so FP64 accuracy from complex64 amplitudes
-// comes from FP32 numbers (AccLevels): a product of two is p + e exactly
-// (e = fma(a, b, -p)); p is split on two fixed grids by adding it to running
-// sums that are held near 1.5 2^k (the sum's own rounding cuts p at 2^(k-23),
-// and the cut-off part comes out exactly), k from the largest components that
-// the two rows have in this chunk, so that kLevelFold steps cannot leave the
-// binade; what is left below 2^(k-41) and e go into a plain FP32 sum whose
-// rounding is the only error.  Every kLevelFold steps the sums are added to
-// FP64.  Amplitudes outside 2^-30 .. 2^60, infinities and NaN, and sums of
-// fewer than kLevelMinK events (which gain nothing) take the FP64 accumulators.
+// and SM against 128 FP32 ones: in FP64 the triangle of 87 waves needs 3.7 ms
+// per 150,000 events, whatever the loads do.
 constexpr int kTriThreads = 256;
-constexpr int kLevelFold = 16;
-constexpr uint64_t kLevelMinK = 4096;
-
-// packed FP32 pairs
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b)
-{
-	float2 d;
-	asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-	    "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-	    : "=f"(d.x), "=f"(d.y)
-	    : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-	return d;
-}
-__device__ __forceinline__ float2 fsub2(float2 a, float2 b)
-{
-	float2 d;
-	asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-	    "sub.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-	    : "=f"(d.x), "=f"(d.y)
-	    : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-	return d;
-}
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b)
-{
-	float2 d;
-	asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-	    "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-	    : "=f"(d.x), "=f"(d.y)
-	    : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-	return d;
-}
 
 // Staged operands of one step, and the loads of a thread tile (rows of group
-// I, columns of unit J).  AccF32 keeps rows 2h, 2h + 1 of a group side by side
+// I, columns of group J).  AccF32 keeps rows 2h, 2h + 1 of a group side by side
 // (one 16-byte load brings both) and the groups' halves apart, AccF64 the four
-// rows apart, AccLevels (two columns per tile) the rows in order: the lanes of
-// a warp, whose J are consecutive, read consecutive 16-byte pieces.
+// rows apart: the lanes of a warp, whose J are consecutive, read consecutive
+// 16-byte pieces.
 __device__ __forceinline__ float4 ldOp(const float2* p) { return *reinterpret_cast<const float4*>(p); }
 
 // 8 bytes from global to shared memory in the background, or zeros
@@ -203,10 +164,10 @@ struct __align__(16) TriSlot {
 struct AccF32 {
 	typedef float2 Op;
 	typedef float Weight;
-	static constexpr int kCols = 4, kUnroll = 2, kFold = 1 << 30;
+	static constexpr int kUnroll = 2;
 	static constexpr bool kAsync = true;
 	float2 s[4][4];
-	__device__ void init(const unsigned*, int, int, int)
+	__device__ void init()
 	{
 		for (int p = 0; p < 4; ++p)
 			for (int q = 0; q < 4; ++q)
@@ -237,17 +198,16 @@ struct AccF32 {
 			}
 		}
 	}
-	__device__ void fold() {}
 	__device__ double2 result(int p, int q) const { return make_double2(s[p][q].x, s[p][q].y); }
 };
 
 struct AccF64 {
 	typedef double2 Op;
 	typedef double Weight;
-	static constexpr int kCols = 4, kUnroll = 2, kFold = 1 << 30;
+	static constexpr int kUnroll = 2;
 	static constexpr bool kAsync = false;
 	double2 s[4][4];
-	__device__ void init(const unsigned*, int, int, int)
+	__device__ void init()
 	{
 		for (int p = 0; p < 4; ++p)
 			for (int q = 0; q < 4; ++q)
@@ -271,145 +231,17 @@ struct AccF64 {
 				s[p][q].y = fma(a[p].y, b[q].x, fma(-a[p].x, b[q].y, s[p][q].y));
 			}
 	}
-	__device__ void fold() {}
 	__device__ double2 result(int p, int q) const { return s[p][q]; }
 };
-
-// two columns per thread tile, so that the three FP32 sums and the FP64 one
-// of its eight elements stay in registers
-struct AccLevels {
-	typedef float2 Op;
-	typedef float Weight;
-	static constexpr int kCols = 2, kUnroll = 4, kFold = kLevelFold;
-	static constexpr bool kAsync = true;
-	float2 s[4][2], u[4][2], c[4][2];  // on the two grids, below them
-	double2 d[4][2];
-	int eRow[4], eCol[2];  // components of the row are below 2^e
-	// sums start at 1.5 2^k with k = eRow + eCol + 6: 2 kLevelFold products
-	// below 2^(k-6) stay below 2^(k-1), their parts cut off at 2^(k-24)
-	// below 2^(k-19), so the second sum starts at 1.5 2^(k-18)
-	static_assert(kLevelFold == 16, "exponents of the running sums");
-	__device__ __forceinline__ float2 start(int p, int q, int drop) const
-	{
-		const float v = __int_as_float(((eRow[p] + eCol[q] + 6 - drop + 127) << 23) | 0x400000);
-		return make_float2(v, v);
-	}
-	__device__ void init(const unsigned* rowMax, int W, int row, int col)
-	{
-		auto expo = [&](int w) { return rowMax && w < W && rowMax[w] ? (int)(rowMax[w] >> 23) - 126 : -29; };
-		for (int p = 0; p < 4; ++p)
-			eRow[p] = expo(row + p);
-		for (int q = 0; q < 2; ++q)
-			eCol[q] = expo(col + q);
-		for (int p = 0; p < 4; ++p)
-			for (int q = 0; q < 2; ++q) {
-				s[p][q] = start(p, q, 0);
-				u[p][q] = start(p, q, 18);
-				c[p][q] = make_float2(0.f, 0.f);
-				d[p][q] = make_double2(0., 0.);
-			}
-	}
-	static __device__ __forceinline__ int pos(int, int row) { return row; }
-	// na = -a
-	static __device__ __forceinline__ void mac(float2 a, float2 na, float2 b, float2& s, float2& u, float2& c)
-	{
-		const float2 p = fmul2(a, b), ne = ffma2(na, b, p);  // a b = p - ne
-		const float2 t = fadd2(s, p), l = fsub2(p, fsub2(t, s));
-		const float2 v = fadd2(u, l), r = fsub2(l, fsub2(v, u));
-		s = t;
-		u = v;
-		c = fsub2(fadd2(c, r), ne);
-	}
-	template <bool WT>
-	__device__ void step(const float2* A, const float2* B, int, int I, int J, float w)
-	{
-		const float4 x = ldOp(A + 4 * I), y = ldOp(A + 4 * I + 2), z = ldOp(B + 2 * J);
-		float2 a[4] = {make_float2(x.x, x.y), make_float2(x.z, x.w), make_float2(y.x, y.y), make_float2(y.z, y.w)};
-		const float2 b[2] = {make_float2(z.x, z.y), make_float2(z.z, z.w)};
-#pragma unroll
-		for (int p = 0; p < 4; ++p) {
-			if (WT)  // 0 or 1
-				a[p] = make_float2(a[p].x * w, a[p].y * w);
-			const float2 na = make_float2(-a[p].x, -a[p].y);
-			const float2 ar = make_float2(a[p].y, na.x), nar = make_float2(na.y, a[p].x);
-#pragma unroll
-			for (int q = 0; q < 2; ++q) {
-				mac(ar, nar, make_float2(b[q].y, b[q].y), s[p][q], u[p][q], c[p][q]);
-				mac(a[p], na, make_float2(b[q].x, b[q].x), s[p][q], u[p][q], c[p][q]);
-			}
-		}
-	}
-	// FP32 to FP64 by integer operations on the fields (the conversion
-	// instruction would occupy the FP64 pipe as long as the addition does);
-	// t is finite, and a subnormal t may come out wrong by 2^-126
-	static __device__ __forceinline__ double widen(float t)
-	{
-		const unsigned b = __float_as_uint(t), m = b & 0x7fffffffu;
-		const double v = __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
-		return m ? v : 0.;
-	}
-	__device__ void fold()
-	{
-#pragma unroll
-		for (int p = 0; p < 4; ++p)
-#pragma unroll
-			for (int q = 0; q < 2; ++q) {
-				const float2 s0 = start(p, q, 0), u0 = start(p, q, 18);
-				const float2 x = fsub2(s[p][q], s0), y = fsub2(u[p][q], u0);
-				// y + c rounded goes with x, the rest of c stays
-				const float2 z = fadd2(y, c[p][q]);
-				c[p][q] = fsub2(c[p][q], fsub2(z, y));
-				d[p][q].x += widen(x.x);
-				d[p][q].y += widen(x.y);
-				d[p][q].x += widen(z.x);
-				d[p][q].y += widen(z.y);
-				s[p][q] = s0;
-				u[p][q] = u0;
-			}
-	}
-	__device__ double2 result(int p, int q) const
-	{
-		return make_double2(d[p][q].x + (double)c[p][q].x, d[p][q].y + (double)c[p][q].y);
-	}
-};
-
-// rowMax[chunk][row] = largest |re|, |im| of the row in the chunk as float
-// bits; *outside is set when one is neither 0 nor in [2^-30, 2^60) (uint order
-// of |x| equals float order; infinities and NaN are above).  A warp per chunk
-// and row.
-__global__ void __launch_bounds__(256) rowMaxKernel(const float2* __restrict__ a, uint64_t n, uint64_t ld,
-                                                    uint64_t chunkLen, int chunks, unsigned* rowMax, unsigned* outside)
-{
-	const int lane = threadIdx.x & 31, chunk = blockIdx.x * 8 + (threadIdx.x >> 5);
-	if (chunk >= chunks)
-		return;
-	const float2* row = a + (uint64_t)blockIdx.y * ld;
-	const uint64_t k0 = (uint64_t)chunk * chunkLen, k1 = min(n, k0 + chunkLen);
-	unsigned m = 0u;
-#pragma unroll 8
-	for (uint64_t k = k0 + lane; k < k1; k += 32) {
-		const float2 v = row[k];
-		m = max(m, max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu));
-	}
-	m = __reduce_max_sync(0xffffffffu, m);
-	if (lane == 0) {
-		rowMax[(size_t)chunk * gridDim.y + blockIdx.y] = m;
-		if (m != 0u && (m < 0x30800000u || m >= 0x5d800000u))
-			*outside = 1u;
-	}
-}
 
 struct TriArgs {
 	uint64_t K, ldK, chunkLen;
 	int W, g;              // rows, groups of four
-	int nTiles;            // thread tiles: groups of four columns g (g + 1) / 2, of two g (g + 1)
+	int nTiles;            // thread tiles: g (g + 1) / 2
 	int tilesPerSlice;     // thread tiles of a slice in one block
 	int slices, chunks;    // chunks of K side by side in a block; chunks in all
 	const double* weightK;
 	double* partials;
-	const unsigned* rowMax;   // AccLevels: rowMaxKernel's result
-	const unsigned* outside;  // null: run; otherwise run when *outside == runOutside
-	unsigned runOutside;
 };
 
 // One block: `slices` chunks of K, one thread tile per thread.  KT steps of
@@ -424,21 +256,18 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 {
 	typedef typename Acc::Op Op;
 	extern __shared__ __align__(16) unsigned char smemRaw[];
-	if (a.outside && *a.outside != a.runOutside)
-		return;
 	const int tid = threadIdx.x, nThreads = blockDim.x;
 	// thread tile (I, J) of this thread, first group I0 of the block
 	const int sl = tid / a.tilesPerSlice;
 	const int t = blockIdx.x * kTriThreads + (tid - sl * a.tilesPerSlice);
-	constexpr int kUnits = 4 / Acc::kCols;  // column units of a group
 	int I = 0, J = blockIdx.x * kTriThreads;
-	while (J >= kUnits * (a.g - I))
-		J -= kUnits * (a.g - I++);
+	while (J >= a.g - I)
+		J -= a.g - I++;
 	const int I0 = I;
 	J += t - blockIdx.x * kTriThreads;
-	while (I < a.g && J >= kUnits * (a.g - I))
-		J -= kUnits * (a.g - I++);
-	J += kUnits * I;
+	while (I < a.g && J >= a.g - I)
+		J -= a.g - I++;
+	J += I;
 	const bool mine = sl < a.slices && t < a.nTiles;
 	const int G = a.g - I0, rows = 4 * G;        // staged groups and rows
 	// a step's operands are an odd number of 16-byte pieces, so that the KT
@@ -450,8 +279,7 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 	Op* const buf0 = reinterpret_cast<Op*>(smemRaw);
 	const uint64_t chunk0 = (uint64_t)blockIdx.y * (unsigned)a.slices;
 	Acc acc;
-	acc.init(mine && chunk0 + sl < (uint64_t)a.chunks ? a.rowMax + (chunk0 + sl) * a.W : nullptr, a.W, 4 * I,
-	         Acc::kCols * J);
+	acc.init();
 
 	// staged rows (slice, row); their weights as the accumulators take them,
 	// for two rounds
@@ -512,7 +340,7 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 	stage(buf0, 0, 0);
 	arrived();
 	const uint32_t len = (uint32_t)a.chunkLen;
-	int cur = 0, sinceFold = 0;
+	int cur = 0;
 	for (uint32_t kb = 0, round = 0; kb < len; kb += KT, ++round) {
 		const bool more = kb + KT < len;
 		Op* const next = buf0 + (cur ^ 1) * bufOps;
@@ -525,12 +353,7 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 			const typename Acc::Weight* w0 = wbuf + ((round & 1) * a.slices + sl) * KT;
 #pragma unroll Acc::kUnroll
 			for (int q = 0; q < KT; ++q)
-				acc.template step<WT>(a0 + q * ld, b0 + q * ld, G, I - I0, J - kUnits * I0, WT ? w0[q] : 0);
-			sinceFold += KT;
-			if (Acc::kFold < (1 << 30) && (sinceFold == Acc::kFold || !more)) {
-				sinceFold = 0;
-				acc.fold();
-			}
+				acc.template step<WT>(a0 + q * ld, b0 + q * ld, G, I - I0, J - I0, WT ? w0[q] : 0);
 		}
 		if (!Acc::kAsync && more)
 			stage(next, kb + KT, round + 1);
@@ -549,8 +372,8 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 #pragma unroll
 	for (int p = 0; p < 4; ++p)
 #pragma unroll
-		for (int q = 0; q < Acc::kCols; ++q) {
-			const int gi = 4 * I + p, gj = Acc::kCols * J + q;
+		for (int q = 0; q < 4; ++q) {
+			const int gi = 4 * I + p, gj = 4 * J + q;
 			if (gi <= gj && gj < a.W)
 				reinterpret_cast<double2*>(out)[(size_t)gi * a.W + gj] = acc.result(p, q);
 		}
@@ -612,9 +435,9 @@ size_t triSliceBytes(int g, int KT, size_t opBytes, bool weighted)
 
 // most chunks that a block of gramTriKernel holds side by side with KT steps
 // per round; 0 when one does not fit
-int triSlices(int W, int cols, int KT, size_t opBytes, bool weighted)
+int triSlices(int W, int KT, size_t opBytes, bool weighted)
 {
-	const int g = (W + 3) / 4, nt = g * (g + 1) / 2 * (4 / cols);
+	const int g = (W + 3) / 4, nt = g * (g + 1) / 2;
 	const size_t one = triSliceBytes(g, KT, opBytes, weighted);
 	if (one > kTriSmemMax)
 		return 0;
@@ -624,11 +447,11 @@ int triSlices(int W, int cols, int KT, size_t opBytes, bool weighted)
 template <typename Acc, typename In, int KT, bool WT>
 int launchTriT(const In* amps, TriArgs t, cudaStream_t s)
 {
-	t.nTiles = t.g * (t.g + 1) / 2 * (4 / Acc::kCols);
+	t.nTiles = t.g * (t.g + 1) / 2;
 	const int blocksX = (t.nTiles + kTriThreads - 1) / kTriThreads;
 	// chunks side by side only where the grid keeps two blocks for each of
 	// the 152 SMs
-	t.slices = std::max(1, std::min(triSlices(t.W, Acc::kCols, KT, sizeof(typename Acc::Op), WT),
+	t.slices = std::max(1, std::min(triSlices(t.W, KT, sizeof(typename Acc::Op), WT),
 	                                t.chunks * blocksX / 304));
 	t.tilesPerSlice = std::min(t.nTiles, kTriThreads);
 	const size_t smem = t.slices * triSliceBytes(t.g, KT, sizeof(typename Acc::Op), WT);
@@ -648,7 +471,7 @@ template <typename Acc, typename In>
 int launchTri(const In* amps, const TriArgs& t, cudaStream_t s)
 {
 	static_assert(sizeof(TriSlot) == 16, "row table entry");
-	const bool wide = triSlices(t.W, Acc::kCols, 16, sizeof(typename Acc::Op), t.weightK != nullptr) == 0;
+	const bool wide = triSlices(t.W, 16, sizeof(typename Acc::Op), t.weightK != nullptr) == 0;
 	if (t.weightK)
 		return wide ? launchTriT<Acc, In, 8, true>(amps, t, s) : launchTriT<Acc, In, 16, true>(amps, t, s);
 	return wide ? launchTriT<Acc, In, 8, false>(amps, t, s) : launchTriT<Acc, In, 16, false>(amps, t, s);
@@ -656,13 +479,7 @@ int launchTri(const In* amps, const TriArgs& t, cudaStream_t s)
 
 bool triFits(int W, int precision, bool weighted)
 {
-	return triSlices(W, 4, 8, precision == 0 ? sizeof(double2) : sizeof(float2), weighted) > 0;
-}
-
-// complex64 rows without weights other than 0 and 1
-bool levelsApply(const GramArgs& a, int precision)
-{
-	return precision == 0 && !a.amps64 && a.rowMax && a.K >= kLevelMinK && (!a.weightK || a.weights01);
+	return triSlices(W, 8, precision == 0 ? sizeof(double2) : sizeof(float2), weighted) > 0;
 }
 
 }  // namespace
@@ -699,19 +516,6 @@ int launchGramSimt(const GramArgs& a, int precision, cudaStream_t s)
 			return launchTri<AccF32, float2>(a.amps, t, s);
 		if (a.amps64)
 			return launchTri<AccF64, double2>(a.amps64, t, s);
-		if (levelsApply(a, precision)) {
-			// both kernels are launched; the amplitudes' range decides on the
-			// device which of them runs
-			t.outside = a.rowMax;
-			PWA_CHECK(cudaCheck(cudaMemsetAsync(a.rowMax, 0, sizeof(unsigned), s), "memset"));
-			t.rowMax = a.rowMax + 1;
-			rowMaxKernel<<<dim3((a.chunks + 7) / 8, a.W), 256, 0, s>>>(a.amps, a.K, a.ldK, chunkLen, a.chunks,
-			                                                          a.rowMax + 1, a.rowMax);
-			countLaunches(1);
-			PWA_CHECK(cudaCheck(cudaGetLastError(), "row range launch"));
-			PWA_CHECK((launchTri<AccLevels, float2>(a.amps, t, s)));
-			t.runOutside = 1;
-		}
 		return launchTri<AccF64, float2>(a.amps, t, s);
 	}
 	const int tps = (a.W + kTile - 1) / kTile;

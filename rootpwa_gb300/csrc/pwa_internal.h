@@ -160,11 +160,6 @@ struct GramArgs {
 	// tensor-core Gram only: 0, or the element offset between two groups of
 	// W / 2 rows each (the Gram of rows 0..W/2-1 and groupStride.. + W/2-1)
 	uint64_t groupStride;
-	// SIMT FP64 Gram of complex64 rows only: scratch of 1 + chunks x W words for
-	// the rows' range (null: FP64 arithmetic throughout), and whether every
-	// weight is 0 or 1
-	unsigned* rowMax;
-	bool weights01;
 };
 // chunks of K for launchGramSimt on a GPU of numSMs (K, W, weightK set)
 int gramSimtChunks(const GramArgs& a, int precision, int numSMs);
