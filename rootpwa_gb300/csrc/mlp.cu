@@ -325,18 +325,23 @@ __global__ void mseKernel(const float* Y, const float* T, int n, int N, int ld16
 // element i of the parameter vector in the padded BF16 weights, or -1 (bias)
 __device__ __forceinline__ long long w16Index(const MlpWeights& w, size_t i)
 {
+	long long o = -1;
 #pragma unroll
-	for (int l = 0; l < 3; ++l)
-		if (i >= w.from[l] && i < w.from[l] + (size_t)w.rows[l] * w.cols[l]) {
-			const size_t q = i - w.from[l];
+	for (int l = 0; l < 3; ++l) {
+		const size_t q = i - w.from[l];  // wraps below the matrix
+		if (q < (size_t)w.rows[l] * w.cols[l]) {
 			const size_t r = q <= 0xffffffffull ? (size_t)((uint32_t)q / (uint32_t)w.cols[l]) : q / w.cols[l];
-			return (long long)(w.to[l] + r * w.ld[l] + (q - r * w.cols[l]));
+			o = (long long)(w.to[l] + r * w.ld[l] + (q - r * w.cols[l]));
 		}
-	return -1;
+	}
+	return o;
 }
 
 // Adam on FP32 master weights; refreshes the BF16 copy.  Four parameters per
-// thread (the arrays come from the allocator, 16-byte aligned).  The moments'
+// thread (the arrays come from the allocator, 16-byte aligned; every index into
+// the thread's own copies is known at compile time, so that they and the
+// weights' map stay in registers: 20 us for 3 M parameters, 24 with the map
+// indexed in local memory).  The moments'
 // fused multiply-adds are written out: a run's weights do not depend on which
 // product the compiler fuses.
 __global__ void __launch_bounds__(256) adamKernel(float* w, const float* __restrict__ g, float* m, float* v,
@@ -348,18 +353,20 @@ __global__ void __launch_bounds__(256) adamKernel(float* w, const float* __restr
 	if (i0 >= n)
 		return;
 	const int k = (int)min((size_t)4, n - i0);
-	float gi[4], mi[4], vi[4], wi[4];
+	alignas(16) float gi[4], mi[4], vi[4], wi[4];
 	if (k == 4) {
 		*reinterpret_cast<float4*>(gi) = *reinterpret_cast<const float4*>(g + i0);
 		*reinterpret_cast<float4*>(mi) = *reinterpret_cast<const float4*>(m + i0);
 		*reinterpret_cast<float4*>(vi) = *reinterpret_cast<const float4*>(v + i0);
 		*reinterpret_cast<float4*>(wi) = *reinterpret_cast<const float4*>(w + i0);
 	} else {
-		for (int j = 0; j < k; ++j) {
-			gi[j] = g[i0 + j];
-			mi[j] = m[i0 + j];
-			vi[j] = v[i0 + j];
-			wi[j] = w[i0 + j];
+#pragma unroll
+		for (int j = 0; j < 4; ++j) {
+			const size_t i = j < k ? i0 + j : i0;
+			gi[j] = g[i];
+			mi[j] = m[i];
+			vi[j] = v[i];
+			wi[j] = w[i];
 		}
 	}
 #pragma unroll
@@ -373,14 +380,17 @@ __global__ void __launch_bounds__(256) adamKernel(float* w, const float* __restr
 		*reinterpret_cast<float4*>(v + i0) = *reinterpret_cast<float4*>(vi);
 		*reinterpret_cast<float4*>(w + i0) = *reinterpret_cast<float4*>(wi);
 	} else {
-		for (int j = 0; j < k; ++j) {
-			m[i0 + j] = mi[j];
-			v[i0 + j] = vi[j];
-			w[i0 + j] = wi[j];
-		}
+#pragma unroll
+		for (int j = 0; j < 4; ++j)
+			if (j < k) {
+				m[i0 + j] = mi[j];
+				v[i0 + j] = vi[j];
+				w[i0 + j] = wi[j];
+			}
 	}
-	for (int j = 0; j < k; ++j) {
-		const long long o = w16Index(map, i0 + j);
+#pragma unroll
+	for (int j = 0; j < 4; ++j) {
+		const long long o = j < k ? w16Index(map, i0 + j) : -1;
 		if (o >= 0)
 			o16[o] = __float2bfloat16_rn(wi[j]);
 	}
