@@ -802,20 +802,29 @@ __global__ void __launch_bounds__(kThreadsHL, 1) gramTcHiLoKernel(const __grid_c
 // FP64 sum of the CTAs' partials; assembles the Hermitian matrix (upper
 // triangle from Re and D, lower mirrored, real diagonal).  sym: the first
 // partial is S with Re = (S + S^T) / 2 (the hi/lo kernel).  Order of the sum,
-// the same on every run: 32 sub-sums over CTAs l, l + 32, ..., combined
-// pairwise at distances 16, 8, 4, 2, 1.  A block takes 32 elements of the upper
-// triangle (146 blocks for 96 columns), a thread four of the sub-sums of one
-// element.  What bounds it is the FP64 pipe (eight operations per element and
-// CTA, conversions included: 10 us of its rate for 96 columns); one warp per
-// element spent as much again on the butterfly and waited for one CTA's loads
-// at a time: 28 us, 19 now.
-constexpr int kRedSub = 8;  // threads per element
-__global__ void __launch_bounds__(32 * kRedSub) gramTcReduceKernel(const float* __restrict__ partials, int grid, int W,
-                                                                   int N, int sym, double* out)
+// the same on every run and for every E, S: 32 sub-sums over CTAs l, l + 32,
+// ..., combined pairwise at distances 16, 8, 4, 2, 1.  A block takes E elements
+// of the upper triangle, S threads each, a thread 32 / S of the sub-sums.
+//
+// What bounds it is the FP64 pipe of the SMs that have a block (eight operations
+// per element and CTA, conversions included), so that the elements have to be
+// spread over them: 32 elements x 8 threads are 146 blocks at 96 columns (10 us
+// of the pipe), but 17 at 32 columns with the same 10 us each.  Times per launch
+// over 152 CTAs (hi/lo partials) by columns, events around launches in a row:
+//   columns                    8     16     32     48     64     87     96    128
+//   32 elements x 8 threads  16.4   16.4   18.5   18.5   18.5   18.5   18.5   30.8 us
+//   4 elements x 32 threads   6.2    6.2    6.6    8.3   12.4   18.5   20.5   30.8
+//   warp per element          8.3    8.2    8.3   12.4   20.5   28.7   28.8   36.9
+template <int E, int S>
+__global__ void __launch_bounds__(E * S) gramTcReduceKernel(const float* __restrict__ partials, int grid, int W, int N,
+                                                            int sym, double* out)
 {
-	__shared__ double sRe[kRedSub][32], sIm[kRedSub][32];
-	const int lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
-	int i = 0, j = (int)blockIdx.x * 32 + lane;
+	static_assert((S == 8 && E == 32) || (S == 32 && 4 * E <= 32), "sub-sums per thread, final threads in one warp");
+	constexpr int M = 32 / S;              // sub-sums per thread
+	constexpr int kRounds = S == 32 ? 5 : 1;  // CTAs of a sub-sum whose loads are in flight together
+	__shared__ double sRe[S][E], sIm[S][E];
+	const int el = threadIdx.x % E, sub = threadIdx.x / E;
+	int i = 0, j = (int)blockIdx.x * E + el;
 	const bool use = j < W * (W + 1) / 2;
 	if (use) {
 		while (j >= W - i) {
@@ -823,42 +832,79 @@ __global__ void __launch_bounds__(32 * kRedSub) gramTcReduceKernel(const float* 
 			++i;
 		}
 		j += i;
-		double re[4] = {0., 0., 0., 0.}, im[4] = {0., 0., 0., 0.};
-		const size_t step = (size_t)2 * 128 * N, toD = (size_t)128 * N;
-		const float* pij = partials + (size_t)i * N + j;
-		const float* pji = partials + (size_t)j * N + i;
-		for (int c0 = sub; c0 < grid; c0 += 32) {
-			float v[4][4];
-#pragma unroll
-			for (int m = 0; m < 4; ++m) {
-				const size_t o = (size_t)min(c0 + 8 * m, grid - 1) * step;
-				v[m][0] = __ldg(pij + o);
-				v[m][1] = __ldg(pji + o);
-				v[m][2] = __ldg(pij + o + toD);
-				v[m][3] = __ldg(pji + o + toD);
-			}
-#pragma unroll
-			for (int m = 0; m < 4; ++m)
-				if (c0 + 8 * m < grid) {
-					re[m] += sym ? 0.5 * ((double)v[m][0] + (double)v[m][1]) : (double)v[m][0];
-					im[m] += (double)v[m][2] - (double)v[m][3];
-				}
-		}
-		sRe[sub][lane] = (re[0] + re[2]) + (re[1] + re[3]);
-		sIm[sub][lane] = (im[0] + im[2]) + (im[1] + im[3]);
+	} else {
+		j = 0;
 	}
+	double re[M], im[M];
+#pragma unroll
+	for (int m = 0; m < M; ++m)
+		re[m] = im[m] = 0.;
+	const size_t step = (size_t)2 * 128 * N, toD = (size_t)128 * N;
+	const float* pij = partials + (size_t)i * N + j;
+	const float* pji = partials + (size_t)j * N + i;
+	for (int c0 = sub; c0 < grid; c0 += 32 * kRounds) {
+		float v[kRounds * M][4];
+#pragma unroll
+		for (int k = 0; k < kRounds * M; ++k) {
+			const int c = c0 + S * k;
+			if (S == 8 || c < grid) {
+				const size_t o = (size_t)min(c, grid - 1) * step;
+				v[k][0] = __ldg(pij + o);
+				v[k][1] = __ldg(pji + o);
+				v[k][2] = __ldg(pij + o + toD);
+				v[k][3] = __ldg(pji + o + toD);
+			}
+		}
+#pragma unroll
+		for (int k = 0; k < kRounds * M; ++k)
+			if (c0 + S * k < grid) {
+				re[k % M] += sym ? 0.5 * ((double)v[k][0] + (double)v[k][1]) : (double)v[k][0];
+				im[k % M] += (double)v[k][2] - (double)v[k][3];
+			}
+	}
+	if constexpr (M == 4) {
+		re[0] = (re[0] + re[2]) + (re[1] + re[3]);
+		im[0] = (im[0] + im[2]) + (im[1] + im[3]);
+	}
+	sRe[sub][el] = re[0];
+	sIm[sub][el] = im[0];
 	__syncthreads();
+	// the first S / 8 threads of each element combine eight sums each
+	if (sub >= S / 8)
+		return;
+	auto tree = [&](const double(*v)[E]) {
+		const auto at = [&](int k) { return v[sub + k * (S / 8)][el]; };
+		double t = ((at(0) + at(4)) + (at(2) + at(6))) + ((at(1) + at(5)) + (at(3) + at(7)));
+		if constexpr (S == 32) {
+			constexpr unsigned lanes = 4 * E == 32 ? 0xffffffffu : (1u << (4 * E % 32)) - 1u;
+			t += __shfl_xor_sync(lanes, t, 2 * E);
+			t += __shfl_xor_sync(lanes, t, E);
+		}
+		return t;
+	};
+	const double r = tree(sRe), d = tree(sIm);
 	if (!use || sub > 0)
 		return;
-	auto tree = [&](const double(*v)[32]) {
-		return ((v[0][lane] + v[4][lane]) + (v[2][lane] + v[6][lane])) +
-		       ((v[1][lane] + v[5][lane]) + (v[3][lane] + v[7][lane]));
-	};
-	const double re = tree(sRe), im = i == j ? 0. : tree(sIm);
-	out[((size_t)i * W + j) * 2] = re;
-	out[((size_t)i * W + j) * 2 + 1] = im;
-	out[((size_t)j * W + i) * 2] = re;
-	out[((size_t)j * W + i) * 2 + 1] = -im;
+	const double q = i == j ? 0. : d;
+	out[((size_t)i * W + j) * 2] = r;
+	out[((size_t)i * W + j) * 2 + 1] = q;
+	out[((size_t)j * W + i) * 2] = r;
+	out[((size_t)j * W + i) * 2 + 1] = -q;
+}
+
+// 4 elements x 32 threads until 32 x 8 give blocks for three quarters of the
+// SMs (85 columns; the two are equal at 87).  With 32 CTAs or fewer a
+// sub-sum is one CTA, and the wide form is ahead from 49 columns on (20
+// CTAs: 8.2 us against 8.2 at 48 columns, 10.3 at 64 and 14.4 at 87).
+int launchGramTcReduce(const float* partials, int grid, int W, int N, int sym, int numSMs, double* out, cudaStream_t s)
+{
+	const int n = W * (W + 1) / 2;
+	if (n >= 24 * numSMs || (grid <= 32 && n >= 8 * numSMs))
+		gramTcReduceKernel<32, 8><<<(n + 31) / 32, 256, 0, s>>>(partials, grid, W, N, sym, out);
+	else
+		gramTcReduceKernel<4, 32><<<(n + 3) / 4, 128, 0, s>>>(partials, grid, W, N, sym, out);
+	countLaunches(1);
+	return cudaCheck(cudaGetLastError(), "gram TC reduce launch");
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -986,10 +1032,7 @@ int launchGramTc(const GramArgs& g, int precision, int numSMs, cudaStream_t s, d
 	}
 	countLaunches(1);
 	PWA_CHECK_RET(cudaCheck(cudaGetLastError(), "gram TC launch"));
-	gramTcReduceKernel<<<(g.W * (g.W + 1) / 2 + 31) / 32, 32 * kRedSub, 0, s>>>(a.partials, grid, g.W, a.N, hiLo ? 1 : 0,
-	                                                                            out);
-	countLaunches(1);
-	return cudaCheck(cudaGetLastError(), "gram TC reduce launch");
+	return launchGramTcReduce(a.partials, grid, g.W, a.N, hiLo ? 1 : 0, numSMs, out, s);
 }
 
 }  // namespace pwa
