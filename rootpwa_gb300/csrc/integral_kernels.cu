@@ -381,11 +381,15 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 
 // Sums chunk partials (upper triangle) in FP64 and writes the full Hermitian
 // matrix; the diagonal's imaginary part is exactly zero as in the reference.
-// A block holds 32 neighbouring elements x 16 slices of the chunks: the 512
-// bytes of a chunk's 32 elements are read together and the loads of a thread
-// are independent (one thread per element, adding one chunk after the other,
-// took 147 us for 203 chunks of 87 waves).
-constexpr int kRedElems = 32, kRedSlices = 16;
+// A block holds 8 neighbouring elements x 16 slices of the chunks: the 128
+// bytes of a chunk's 8 elements are read together and the loads of a thread are
+// independent.  Order of the sum, the same on every run: slice y adds chunks
+// y, y + 16, ... in order, then the slices are added in order.  What bounds it
+// is the FP64 pipe of the SMs that have a block: 8 elements each rather than 32
+// take 24.6 us instead of 51.3 for 5 to 24 waves and 2,432 chunks, 10.3 instead
+// of 16.4 for 5 to 32 waves and 608, 14.4 instead of 16.4 for 87 waves and 304
+// (one thread per element, chunk after chunk: 252 to 382, 66 to 98 and 51 us).
+constexpr int kRedElems = 8, kRedSlices = 16;
 __global__ void __launch_bounds__(kRedElems * kRedSlices) gramReduceKernel(const double* partials, int chunks, int W,
                                                                           double* out, int accumulate)
 {
