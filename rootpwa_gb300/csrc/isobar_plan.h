@@ -142,9 +142,12 @@ inline std::string checkWave(const pwa_isobar_wave& w, bool reflBasis)
 // Helicity formalism: dPlus/dMinus = d^J_{+-M lam}, dIso = d^j_{lam 0}.
 // Canonical formalism: dPlus/dMinus = d^L_{+-M-m, 0} (spherical harmonics
 // Y_L), dIso = d^l_{m 0}, and the whole times e^{-i m phi/2}.
+struct DRange {
+	int32_t at = 0, n = 0;          // terms of a d function in Plan::dterms
+};
 struct LamTerm {
 	int32_t lamIso;                 // 2 lambda (helicity) or 2 m (canonical) of the isobar
-	std::vector<DTerm> plus, minus, iso;  // minus empty if unused
+	DRange plus, minus, iso;        // minus empty if unused
 	double cPlus, cMinus;
 };
 
@@ -158,7 +161,7 @@ struct Term {
 // a wave as buildPlan collects it, before compilePlan
 struct WaveSource {
 	int32_t J, M;
-	std::vector<LamTerm> lams;
+	int32_t lam0, lam1;             // range in Plan::lamTerms
 	std::vector<std::pair<int, double>> terms;  // (permutation index, factor)
 	int32_t iso;                    // first wave of its isobar class
 };
@@ -166,6 +169,8 @@ struct WaveSource {
 struct Plan {
 	std::vector<WaveDev> waves;
 	std::vector<WaveSource> source;
+	std::vector<LamTerm> lamTerms;
+	std::vector<DTerm> dterms;
 	std::vector<Batch> batches;
 	std::vector<int32_t> insts, isoWave, phaseM, lxL;
 	std::vector<EOp> eops;
@@ -271,7 +276,10 @@ constexpr int kMaxTable = 640;
 // Compiles the collected waves into batches (isobar_math.cuh).  The waves of
 // one topology class are taken family by family -- helicity formalism: equal
 // J and |M|; canonical: equal X-vertex L -- and within a family by angular
-// sum; a batch is closed when the next wave's entries would not fit.
+// sum; a batch is closed when the next wave's entries would not fit (the batch
+// is then collected again without it, which almost never happens: a copy of the
+// batch per wave made buildPlan take 1,070 us for 88 waves where it takes 120,
+// 32 of them here; an object compiles its plan in its first call).
 class PlanCompiler {
 public:
 	explicit PlanCompiler(Plan& p) : P(p) {}
@@ -317,13 +325,13 @@ private:
 	};
 	struct Fam {
 		std::pair<int, int> key;
-		std::vector<std::vector<DTerm>> ds;
+		std::vector<DRange> ds;
 		std::vector<XOp<double>> xs;  // phase: 2M
 		std::vector<Ang> angs;
 	};
 	struct Draft {
 		std::vector<int> insts, isos, phases, ls;
-		std::vector<std::pair<int, std::vector<DTerm>>> es;  // (2 lam, d function)
+		std::vector<std::pair<int, DRange>> es;  // (2 lam, d function)
 		std::vector<Fam> fams;
 		int pow = 0;
 		int size() const
@@ -365,12 +373,13 @@ private:
 	}
 	// +1 or -1 when y is x or -x term by term, else 0 (the same function from
 	// another formula may differ in the last bits of its coefficients)
-	static int sameD(const std::vector<DTerm>& x, const std::vector<DTerm>& y)
+	int sameD(DRange rx, DRange ry) const
 	{
-		if (x.size() != y.size())
+		if (rx.n != ry.n)
 			return 0;
+		const DTerm *x = P.dterms.data() + rx.at, *y = P.dterms.data() + ry.at;
 		int s = 0;
-		for (size_t i = 0; i < x.size(); ++i) {
+		for (int i = 0; i < rx.n; ++i) {
 			if (x[i].a != y[i].a || x[i].b != y[i].b)
 				return 0;
 			const int si = std::fabs(x[i].coef - y[i].coef) <= 1e-14 * std::fabs(x[i].coef)   ? 1
@@ -382,15 +391,15 @@ private:
 		}
 		return s;
 	}
-	static int powerOf(const std::vector<DTerm>& t)
+	int powerOf(DRange t) const
 	{
 		int p = 0;
-		for (const DTerm& d : t)
-			p = std::max(p, std::max(d.a, d.b));
+		for (int i = t.at; i < t.at + t.n; ++i)
+			p = std::max(p, std::max(P.dterms[i].a, P.dterms[i].b));
 		return p;
 	}
 	// entry of the d function in its family, and the sign it comes with
-	static int findD(Fam& f, const std::vector<DTerm>& t, double* sign)
+	int findD(Fam& f, DRange t, double* sign) const
 	{
 		for (size_t i = 0; i < f.ds.size(); ++i) {
 			const int s = sameD(f.ds[i], t);
@@ -415,7 +424,7 @@ private:
 		f.xs.push_back(x);
 		return (int)f.xs.size() - 1;
 	}
-	int findE(Draft& d, int lam, const std::vector<DTerm>& t) const
+	int findE(Draft& d, int lam, DRange t) const
 	{
 		for (size_t i = 0; i < d.es.size(); ++i)
 			if (d.es[i].first == lam && sameD(d.es[i].second, t) == 1)
@@ -445,23 +454,25 @@ private:
 		}
 		Ang a;
 		a.L = P.waves[w].LX;
-		for (const LamTerm& l : src.lams) {
+		a.lams.reserve(src.lam1 - src.lam0);
+		for (int k = src.lam0; k < src.lam1; ++k) {
+			const LamTerm& l = P.lamTerms[k];
 			XOp<double> x{};
 			LamOp<double> op{};
 			double cP = 0.0, cM = 0.0, s = 1.0;
-			if (!l.plus.empty()) {
+			if (l.plus.n > 0) {
 				x.dP = findD(*f, l.plus, &s);
 				cP = s * l.cPlus;
 				d.pow = std::max(d.pow, powerOf(l.plus));
 			}
-			if (!l.minus.empty()) {
+			if (l.minus.n > 0) {
 				x.dM = findD(*f, l.minus, &s);
 				cM = s * l.cMinus;
 				d.pow = std::max(d.pow, powerOf(l.minus));
 			}
-			if (l.plus.empty())
+			if (l.plus.n == 0)
 				x.dP = x.dM;
-			if (l.minus.empty())
+			if (l.minus.n == 0)
 				x.dM = x.dP;
 			x.phase = src.M;
 			x.a = cP != 0.0 ? 1.0 : 0.0;
@@ -483,37 +494,44 @@ private:
 				return;
 			}
 		a.waves.push_back(w);
-		f->angs.push_back(a);
+		f->angs.push_back(std::move(a));
 	}
 
 	void topology(std::vector<int> waves)
 	{
 		std::stable_sort(waves.begin(), waves.end(), [&](int x, int y) { return family(x) < family(y); });
+		std::vector<int> mine;  // the waves of d
 		Draft d;
-		bool any = false;
 		for (int w : waves) {
-			Draft next = d;
-			add(next, w);
-			if (any && next.size() > kMaxTable) {
-				emit(d);
-				next = Draft();
-				add(next, w);
+			add(d, w);
+			if (!mine.empty() && d.size() > kMaxTable) {
+				// one too many: the batch again without it, and a new one
+				emit(draftOf(mine));
+				mine.clear();
+				d = draftOf({w});
 			}
-			d = next;
-			any = true;
+			mine.push_back(w);
 		}
 		emit(d);
 	}
 
-	DOp dop(const std::vector<DTerm>& t)
+	Draft draftOf(const std::vector<int>& waves) const
+	{
+		Draft d;
+		for (int w : waves)
+			add(d, w);
+		return d;
+	}
+
+	DOp dop(DRange t)
 	{
 		DOp o{};
 		o.coef0 = (int32_t)P.coef.size();
-		o.n = (int32_t)t.size();
-		o.c = t.back().a;
-		o.s = t.front().b;
-		for (const DTerm& x : t)
-			P.coef.push_back(x.coef);
+		o.n = t.n;
+		o.c = P.dterms[t.at + t.n - 1].a;
+		o.s = P.dterms[t.at].b;
+		for (int i = t.at; i < t.at + t.n; ++i)
+			P.coef.push_back(P.dterms[i].coef);
 		P.coef.resize((P.coef.size() + 3) / 4 * 4, 0.0);
 		return o;
 	}
@@ -564,7 +582,7 @@ private:
 		for (const Fam& f : d.fams) {
 			FamOp F{};
 			F.d0 = (int32_t)P.dops.size();
-			for (const auto& t : f.ds)
+			for (DRange t : f.ds)
 				P.dops.push_back(dop(t));
 			F.d1 = (int32_t)P.dops.size();
 			F.x0 = (int32_t)P.xops.size();
@@ -783,13 +801,23 @@ inline std::vector<Term> symTerms(const pwa_isobar_wave& w, const int32_t specie
 	return out;
 }
 
+// d^j_{m n} appended to the plan's terms
+inline DRange addWigner(int j, int m, int n, Plan& plan)
+{
+	DRange r;
+	r.at = (int32_t)plan.dterms.size();
+	wignerTerms(j, m, n, plan.dterms);
+	r.n = (int32_t)plan.dterms.size() - r.at;
+	return r;
+}
+
 // canonical formalism (isobarCanonicalAmplitude::twoBodyDecayAmplitude,
 // isobarCanonicalAmplitude.cc:118-190): for each spin projection m of the
 // isobar, X vertex sqrt(4 pi) (s1 m1 s2 m2 | S m) F_L sum_mL C(mL) Y_L^mL and
 // isobar vertex sqrt(4 pi) (0 0 0 0 | S' 0) F_l (l m S' 0 | j m) Y_l^m.  The
 // (L mL S m | J +-M) couplings vanish unless mL = +-M - m, so the sum over mL
 // keeps two terms; sqrt(4 pi) Y_L^mu = sqrt(2L+1) e^{i mu phi} d^L_{mu 0}.
-inline void addCanonicalTerms(const pwa_isobar_wave& s, bool reflBasis, std::vector<LamTerm>& lams)
+inline void addCanonicalTerms(const pwa_isobar_wave& s, bool reflBasis, Plan& plan)
 {
 	const int J = s.J, M = s.M, L = s.L, S = s.S, j = s.isobarJ, l = s.isobarL, Si = s.isobarS;
 	for (int m = -j; m <= j; m += 2) {
@@ -823,13 +851,13 @@ inline void addCanonicalTerms(const pwa_isobar_wave& s, bool reflBasis, std::vec
 		LamTerm t{};
 		t.lamIso = m;
 		if (cP != 0.0)
-			wignerTerms(L, mP, 0, t.plus);
+			t.plus = addWigner(L, mP, 0, plan);
 		if (cM != 0.0)
-			wignerTerms(L, mM, 0, t.minus);
-		wignerTerms(l, m, 0, t.iso);
+			t.minus = addWigner(L, mM, 0, plan);
+		t.iso = addWigner(l, m, 0, plan);
 		t.cPlus = c * cP;
 		t.cMinus = c * cM;
-		lams.push_back(t);
+		plan.lamTerms.push_back(t);
 	}
 }
 
@@ -854,6 +882,8 @@ inline std::string buildPlan(const std::vector<pwa_isobar_wave>& specs, const do
 	plan.reflection = reflection ? 1 : 0;
 	plan.waves.clear();
 	plan.source.clear();
+	plan.lamTerms.clear();
+	plan.dterms.clear();
 	barrierPolynomials(plan.bfPoly, plan.bfNorm);
 	plan.perms.clear();
 	{
@@ -909,8 +939,9 @@ inline std::string buildPlan(const std::vector<pwa_isobar_wave>& specs, const do
 				wMinus = -f / std::sqrt(2.0);
 			}
 		}
+		src.lam0 = (int32_t)plan.lamTerms.size();
 		if (canonical)
-			addCanonicalTerms(s, reflBasis, src.lams);
+			addCanonicalTerms(s, reflBasis, plan);
 		for (int lamIso = -s.isobarJ; lamIso <= s.isobarJ && !zero && !canonical; lamIso += 2) {
 			// X -> daughter 1 + daughter 2 with helicities (l1, l2), spins (s1, s2)
 			const int s1 = s.bachelorFirst ? 0 : s.isobarJ, l1 = s.bachelorFirst ? 0 : lamIso;
@@ -926,16 +957,17 @@ inline std::string buildPlan(const std::vector<pwa_isobar_wave>& specs, const do
 			const double c = std::sqrt(s.L + 1.0) * cgX * std::sqrt(s.isobarL + 1.0) * cgI;
 			LamTerm t{};
 			t.lamIso = lamIso;
-			wignerTerms(s.J, s.M, lam, t.plus);
+			t.plus = addWigner(s.J, s.M, lam, plan);
 			if (wMinus != 0.0)
-				wignerTerms(s.J, -s.M, lam, t.minus);
-			wignerTerms(s.isobarJ, lamIso, 0, t.iso);
+				t.minus = addWigner(s.J, -s.M, lam, plan);
+			t.iso = addWigner(s.isobarJ, lamIso, 0, plan);
 			t.cPlus = c * wPlus;
 			t.cMinus = c * wMinus;
-			src.lams.push_back(t);
+			plan.lamTerms.push_back(t);
 		}
+		src.lam1 = (int32_t)plan.lamTerms.size();
 		plan.waves.push_back(w);
-		plan.source.push_back(src);
+		plan.source.push_back(std::move(src));
 	}
 	// isobar classes: waves whose mass dependence (kind and parameters) and
 	// isobar barrier factor agree share their product per event and term
