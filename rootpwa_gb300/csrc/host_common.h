@@ -141,8 +141,13 @@ using namespace pwa;
 // ===========================================================================
 // device buffers and stream of integrate(), kept by an integral between
 // calls on one device (the output matrix, the error flag, the Gram partials
-// and the event weights: no allocation per call once they have their size)
+// and up to kKeepWeights of event weights: no allocation per call once they
+// have their size)
 struct GramScratch {
+	// weights and inverse weights of four million events; above that they are
+	// given back after the call, which costs 0.29 ms of it (8 waves x 3 M events:
+	// 0.93 ms per call with the weights kept, 1.21 without)
+	static constexpr size_t kKeepWeights = size_t(64) << 20;
 	int dev = -1;
 	cudaStream_t stream = nullptr;
 	DevBuf out, err, part, weights, rawWeights;
@@ -150,6 +155,13 @@ struct GramScratch {
 	GramScratch(const GramScratch&) = delete;
 	GramScratch& operator=(const GramScratch&) = delete;
 	~GramScratch() { reset(); }
+	void trim()
+	{
+		if (weights.bytes + rawWeights.bytes > kKeepWeights) {
+			weights.release();
+			rawWeights.release();
+		}
+	}
 	void reset()
 	{
 		out.release();

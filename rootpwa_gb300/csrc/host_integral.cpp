@@ -39,6 +39,10 @@ int gramOnDevice(GramScratch& sc, uint32_t W, const void* amps, uint64_t nEvents
 	// the tensor-core kernel reads rows with TMA: even row stride (16-byte
 	// multiple) and a 16-byte aligned base
 	const uint64_t ldPad = tensorCore ? (K + (K & 1ull)) : K;
+	struct Trim {
+		GramScratch& sc;
+		~Trim() { sc.trim(); }
+	} trim{sc};
 	DevBuf dIn, dConv;
 	DevBuf &dPart = sc.part, &dOut = sc.out, &dErr = sc.err;
 	const float2* a32 = nullptr;
