@@ -206,11 +206,12 @@ __device__ __forceinline__ void fdfTail(const FdfArgs& a, unsigned* sLast, doubl
 // rank 2 144, now 142; 45 waves of rank 3 125, now 118.
 template <int E, int NE>
 struct LaneRoles {
+	static_assert(E == 64 || E == 128, "tiles of 64 or 128 events");
 	__host__ __device__ static constexpr int bit(int i)
 	{
 		return E == 128  ? (i == 0 ? 1 : i == 1 ? 2 : i == 2 ? 0 : i)
-		       : E == 64 ? (NE == 1 ? (i == 3 ? 0 : i < 3 ? i + 1 : i) : (i == 0 ? 3 : i == 3 ? 0 : i))
-		                 : (i == 0 ? 4 : i == 4 ? 0 : i);
+		       : NE == 1 ? (i == 3 ? 0 : i < 3 ? i + 1 : i)
+		                 : (i == 0 ? 3 : i == 3 ? 0 : i);
 	}
 	__device__ static __forceinline__ int role(int lane)
 	{

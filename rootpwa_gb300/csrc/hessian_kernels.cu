@@ -24,8 +24,8 @@ namespace {
 constexpr int kMaxRW = 1024;  // rank x waves held in shared memory
 
 // One event per thread, two passes over its amplitudes: the coherent sums of
-// all ranks together (up to kPrepRanks; more ranks in groups, whose sums the
-// second pass forms again), then the columns.  Bound by the columns' stores
+// all ranks together (at most kPrepRanks, the ranks that the FdF kernels take),
+// then the columns.  Bound by the columns' stores
 // (16 bytes per slot and event plus 8 per wave); a pass per rank and purpose,
 // one load in flight each, took 413 us for 87 waves, rank 2 and 250,001 events
 // (0.88 GB), 214 now.
@@ -43,8 +43,7 @@ struct EventRow {
 	}
 };
 
-__device__ __forceinline__ void coherentSums(const EventRow& amps, const float2* Vs, int W0, int W, int r0, int nR,
-                                             float2 (&S0)[kPrepRanks], float2 (&S1)[kPrepRanks])
+__device__ __forceinline__ void coherentSums(const EventRow& amps, const float2* Vs, int W0, int W, int R, float2 (&S0)[kPrepRanks], float2 (&S1)[kPrepRanks])
 {
 #pragma unroll
 	for (int r = 0; r < kPrepRanks; ++r)
@@ -55,8 +54,8 @@ __device__ __forceinline__ void coherentSums(const EventRow& amps, const float2*
 			const float2 a = amps[w];
 #pragma unroll
 			for (int r = 0; r < kPrepRanks; ++r)
-				if (r < nR) {
-					const float2 v = Vs[(r0 + r) * W + w];
+				if (r < R) {
+					const float2 v = Vs[r * W + w];
 					S[r].x = fmaf(v.x, a.x, fmaf(-v.y, a.y, S[r].x));
 					S[r].y = fmaf(v.x, a.y, fmaf(v.y, a.x, S[r].y));
 				}
@@ -90,44 +89,35 @@ __global__ void __launch_bounds__(256) hessPrepKernel(const float2* __restrict__
 		float2 S0[kPrepRanks], S1[kPrepRanks];
 		// L and f
 		float L = flat2;
-		for (int r0 = 0; r0 < R; r0 += kPrepRanks) {
-			const int nR = min(kPrepRanks, R - r0);
-			coherentSums(row, Vs, W0, W, r0, nR, S0, S1);
+		coherentSums(row, Vs, W0, W, R, S0, S1);
 #pragma unroll
-			for (int r = 0; r < kPrepRanks; ++r)
-				if (r < nR) {
-					L = fmaf(S0[r].x, S0[r].x, fmaf(S0[r].y, S0[r].y, L));
-					L = fmaf(S1[r].x, S1[r].x, fmaf(S1[r].y, S1[r].y, L));
-				}
-		}
+		for (int r = 0; r < kPrepRanks; ++r)
+			if (r < R) {
+				L = fmaf(S0[r].x, S0[r].x, fmaf(S0[r].y, S0[r].y, L));
+				L = fmaf(S1[r].x, S1[r].x, fmaf(S1[r].y, S1[r].y, L));
+			}
 		const float f = valid ? 2.f / L : 0.f;
 		w1[t] = valid ? (double)f * (double)f : 0.;
 		w2[t] = valid ? (double)f : 0.;
 		// d_s, conj(d_s) and the amplitudes
-		for (int r0 = 0; r0 < R; r0 += kPrepRanks) {
-			const int nR = min(kPrepRanks, R - r0);
-			if (R > kPrepRanks)
-				coherentSums(row, Vs, W0, W, r0, nR, S0, S1);
-			auto columns = [&](int from, int to, const float2(&S)[kPrepRanks]) {
+		auto columns = [&](int from, int to, const float2(&S)[kPrepRanks]) {
 #pragma unroll 4
-				for (int w = from; w < to; ++w) {
-					const float2 a = row[w];
+			for (int w = from; w < to; ++w) {
+				const float2 a = row[w];
 #pragma unroll
-					for (int r = 0; r < kPrepRanks; ++r)
-						if (r < nR) {
-							// S conj(a)
-							const float2 d = make_float2(S[r].x * a.x + S[r].y * a.y, S[r].y * a.x - S[r].x * a.y);
-							const size_t k = (size_t)((r0 + r) * W + w);
-							Y1[k * slab + t] = d;
-							Y1[(nS + k) * slab + t] = make_float2(d.x, -d.y);
-						}
-					if (r0 == 0)
-						Y2[(size_t)w * slab + t] = a;
-				}
-			};
-			columns(0, W0, S0);
-			columns(W0, W, S1);
-		}
+				for (int r = 0; r < kPrepRanks; ++r)
+					if (r < R) {
+						// S conj(a)
+						const float2 d = make_float2(S[r].x * a.x + S[r].y * a.y, S[r].y * a.x - S[r].x * a.y);
+						const size_t k = (size_t)(r * W + w);
+						Y1[k * slab + t] = d;
+						Y1[(nS + k) * slab + t] = make_float2(d.x, -d.y);
+					}
+				Y2[(size_t)w * slab + t] = a;
+			}
+		};
+		columns(0, W0, S0);
+		columns(W0, W, S1);
 		Y1[(size_t)(2 * nS) * slab + t] = make_float2(1.f, 0.f);
 		Y2[(size_t)W * slab + t] = make_float2(1.f, 0.f);
 	}
@@ -139,8 +129,8 @@ int launchHessPrep(const float2* amps, uint64_t nEvents, uint32_t B, uint64_t e0
                    int R, int P, const double* par, const int* slotRe, const int* slotIm, float2* Y1, float2* Y2,
                    double* w1, double* w2, cudaStream_t s)
 {
-	if (R * W > kMaxRW)
-		return setError(kErrUnsupported, "Hessian kernel supports rank x waves <= 1024");
+	if (R < 1 || R > kPrepRanks || R * W > kMaxRW)
+		return setError(kErrUnsupported, "Hessian kernel supports rank 1..4 and rank x waves <= 1024");
 	const int threads = 256;
 	const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((slab + threads - 1) / threads, 8192));
 	hessPrepKernel<<<blocks, threads, 0, s>>>(amps, nEvents, B, e0, slab, W0, W, R, P, par, slotRe, slotIm, Y1, Y2,

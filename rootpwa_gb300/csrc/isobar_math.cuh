@@ -43,7 +43,6 @@ namespace iso {
 
 constexpr int kMaxSpin = 16;      // 2J: spins up to 8
 constexpr int kMaxL = 14;         // 2L: barrier factors up to L = 7
-constexpr int kMaxPerms = 6;      // Bose terms of three particles
 constexpr double kPr = 0.1973;    // GeV/c, 1 fm interaction radius
 
 enum {
