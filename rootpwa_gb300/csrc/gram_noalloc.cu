@@ -86,14 +86,15 @@ extern "C" int pwa_gram_device_noalloc(const void* amps, uint64_t nK, uint64_t l
 	double* scratch = nullptr;
 	NOALLOC_TRY(scratchFor(dev, &scratch));
 
-	// integrate()'s chunking: chunks of K per output tile so that the grid
-	// fills the GPU, each a run of chunkLen events summed in the kernel's
-	// accumulator type
+	// integrate()'s chunks of K, each a run of chunkLen events summed in the
+	// kernel's accumulator type
 	const size_t perChunk = (size_t)nWaves * nWaves * 2;
-	const int tps = ((int)nWaves + 63) / 64;
-	const int nTiles = tps * (tps + 1) / 2;
-	uint64_t chunks = (uint64_t)std::max(1, (4 * sms + nTiles - 1) / nTiles);
-	chunks = std::min<uint64_t>(chunks, std::max<uint64_t>(1, nK / 64));
+	const int simt = precision == PWA_PRECISION_FP64 ? 0 : 1;
+	GramArgs whole{};
+	whole.K = nK;
+	whole.W = (int)nWaves;
+	whole.weightK = weights;
+	const uint64_t chunks = (uint64_t)gramSimtChunks(whole, simt, sms);
 	const uint64_t chunkLen = (nK + chunks - 1) / chunks;
 	// the fixed array holds maxChunks chunk partials; a longer input is taken
 	// in segments of maxChunks chunks of the same length, each reduced into
@@ -113,7 +114,7 @@ extern "C" int pwa_gram_device_noalloc(const void* amps, uint64_t nK, uint64_t l
 		g.partials = scratch;
 		g.chunks = (int)((kSeg + chunkLen - 1) / chunkLen);
 		g.devErr = nullptr;
-		NOALLOC_TRY(launchGramSimt(g, precision == PWA_PRECISION_FP64 ? 0 : 1, s));
+		NOALLOC_TRY(launchGramSimt(g, simt, sms, s));
 		NOALLOC_TRY(launchGramReduce(scratch, g.chunks, (int)nWaves, out, seg > 0 ? 1 : 0, s));
 	}
 	return kOk;

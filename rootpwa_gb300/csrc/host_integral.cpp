@@ -147,7 +147,7 @@ int gramOnDevice(GramScratch& sc, uint32_t W, const void* amps, uint64_t nEvents
 		g.chunks = chunks;
 		PWA_TRY(dPart.ensure((size_t)chunks * W * W * 2 * sizeof(double), "gram partials"));
 		g.partials = dPart.as<double>();
-		PWA_TRY(launchGramSimt(g, precision, s));
+		PWA_TRY(launchGramSimt(g, precision, sms, s));
 		PWA_TRY(launchGramReduce(g.partials, chunks, (int)W, dOut.as<double>(), 0, s));
 	}
 	std::vector<double> host(nOut + (rawWeights ? kWeightBlocks : 0));
@@ -593,13 +593,12 @@ int pwa_gram_device_batch(const void* const* amps, const uint64_t* nEvents, uint
 	for (uint32_t b = 0; b < nBins; ++b)
 		nMax = std::max(nMax, nEvents[b]);
 	// partials of the largest bin, reused bin after bin in stream order
-	const int tps = (W + 63) / 64;
-	const int nTiles = tps * (tps + 1) / 2;
 	// SIMT chunks as integrate() takes them, within 256 MiB of FP64 partials
+	GramArgs largest{};
+	largest.K = nMax;
+	largest.W = W;
 	const uint64_t partialBudget = std::max<uint64_t>(1, (256ull << 20) / ((uint64_t)W * W * 2 * sizeof(double)));
-	const int simtChunks = (int)std::min<uint64_t>(
-	    std::min<uint64_t>((uint64_t)std::max(1, (4 * sms + nTiles - 1) / nTiles), std::max<uint64_t>(1, nMax / 64)),
-	    partialBudget);
+	const int simtChunks = (int)std::min<uint64_t>((uint64_t)gramSimtChunks(largest, 1, sms), partialBudget);
 	const size_t tcScratch = tc ? gramTcScratchFloats(W, sms) / 2 + 1 : 0;
 	// tensor-core precisions: bins whose rows are not 16-byte aligned (odd
 	// event count or base) are copied into an aligned buffer of even row
@@ -649,7 +648,7 @@ int pwa_gram_device_batch(const void* const* amps, const uint64_t* nEvents, uint
 			g.ldK = n;
 			g.chunks = (int)std::min<uint64_t>((uint64_t)simtChunks, std::max<uint64_t>(1, n / 64));
 			g.partials = dPart.as<double>();
-			PWA_TRY(launchGramSimt(g, 1, s));
+			PWA_TRY(launchGramSimt(g, 1, sms, s));
 			PWA_TRY(launchGramReduce(g.partials, g.chunks, W, out, 0, s));
 		}
 	}

@@ -449,14 +449,13 @@ int triSlices(int W, int KT, size_t opBytes, bool weighted)
 }
 
 template <typename Acc, typename In, int KT, bool WT>
-int launchTriT(const In* amps, TriArgs t, cudaStream_t s)
+int launchTriT(const In* amps, TriArgs t, int numSMs, cudaStream_t s)
 {
 	t.nTiles = t.g * (t.g + 1) / 2;
 	const int blocksX = (t.nTiles + kTriThreads - 1) / kTriThreads;
-	// chunks side by side only where the grid keeps two blocks for each of
-	// the 152 SMs
+	// chunks side by side only where the grid keeps two blocks for each SM
 	t.slices = std::max(1, std::min(triSlices(t.W, KT, sizeof(typename Acc::Op), WT),
-	                                t.chunks * blocksX / 304));
+	                                t.chunks * blocksX / (2 * numSMs)));
 	t.tilesPerSlice = std::min(t.nTiles, kTriThreads);
 	const size_t smem = t.slices * triSliceBytes(t.g, KT, sizeof(typename Acc::Op), WT);
 	auto kern = gramTriKernel<Acc, In, KT, WT>;
@@ -472,13 +471,14 @@ int launchTriT(const In* amps, TriArgs t, cudaStream_t s)
 }
 
 template <typename Acc, typename In>
-int launchTri(const In* amps, const TriArgs& t, cudaStream_t s)
+int launchTri(const In* amps, const TriArgs& t, int numSMs, cudaStream_t s)
 {
 	static_assert(sizeof(TriSlot) == 16, "row table entry");
 	const bool wide = triSlices(t.W, 16, sizeof(typename Acc::Op), t.weightK != nullptr) == 0;
 	if (t.weightK)
-		return wide ? launchTriT<Acc, In, 8, true>(amps, t, s) : launchTriT<Acc, In, 16, true>(amps, t, s);
-	return wide ? launchTriT<Acc, In, 8, false>(amps, t, s) : launchTriT<Acc, In, 16, false>(amps, t, s);
+		return wide ? launchTriT<Acc, In, 8, true>(amps, t, numSMs, s)
+		            : launchTriT<Acc, In, 16, true>(amps, t, numSMs, s);
+	return wide ? launchTriT<Acc, In, 8, false>(amps, t, numSMs, s) : launchTriT<Acc, In, 16, false>(amps, t, numSMs, s);
 }
 
 bool triFits(int W, int precision, bool weighted)
@@ -503,7 +503,7 @@ int gramSimtChunks(const GramArgs& a, int precision, int numSMs)
 	return (int)std::min<uint64_t>(most, (uint64_t)std::max(1, (4 * numSMs + nTiles - 1) / nTiles));
 }
 
-int launchGramSimt(const GramArgs& a, int precision, cudaStream_t s)
+int launchGramSimt(const GramArgs& a, int precision, int numSMs, cudaStream_t s)
 {
 	const uint64_t chunkLen = ((a.K + a.chunks - 1) / a.chunks + kKT - 1) / kKT * kKT;
 	if (triFits(a.W, precision, a.weightK != nullptr)) {
@@ -517,10 +517,10 @@ int launchGramSimt(const GramArgs& a, int precision, cudaStream_t s)
 		t.weightK = a.weightK;
 		t.partials = a.partials;
 		if (precision != 0)
-			return launchTri<AccF32, float2>(a.amps, t, s);
+			return launchTri<AccF32, float2>(a.amps, t, numSMs, s);
 		if (a.amps64)
-			return launchTri<AccF64, double2>(a.amps64, t, s);
-		return launchTri<AccF64, float2>(a.amps, t, s);
+			return launchTri<AccF64, double2>(a.amps64, t, numSMs, s);
+		return launchTri<AccF64, float2>(a.amps, t, numSMs, s);
 	}
 	const int tps = (a.W + kTile - 1) / kTile;
 	const int nTiles = tps * (tps + 1) / 2;

@@ -163,11 +163,12 @@ struct GramArgs {
 };
 // chunks of K for launchGramSimt on a GPU of numSMs (K, W, weightK set)
 int gramSimtChunks(const GramArgs& a, int precision, int numSMs);
-int launchGramSimt(const GramArgs& a, int precision, cudaStream_t s);
+int launchGramSimt(const GramArgs& a, int precision, int numSMs, cudaStream_t s);
 // out = (accumulate ? out : 0) + sum of chunk partials, mirrored to the lower triangle
 int launchGramReduce(const double* partials, int chunks, int W, double* out, int accumulate, cudaStream_t s);
 // out[ev * nSub + s] = 1 / w[ev] and, per block, the compensated sum of 1 / w
-// of its events into sums[kWeightBlocks]
+// of its events into sums[kWeightBlocks] (a fixed number, so that the sum does
+// not depend on the GPU; one block for each SM of a GB300)
 constexpr int kWeightBlocks = 152;
 int launchInverseWeights(const double* w, uint64_t n, uint32_t nSub, double* out, double* sums, cudaStream_t s);
 // out[w] = sum_k a[w][k] for W complex64 rows of n elements (row stride ld),
