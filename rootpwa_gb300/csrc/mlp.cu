@@ -26,7 +26,7 @@
 // single-element operand loads and one row per lane in the drain; vector
 // loads alone left 12 to 15 us and, for the first layer and its weight
 // gradient, 32 and 44; with rows stored whole, 7 and 13 and 16.  A training
-// step takes 178 us against 352 before (Adam's 83 MB among them: 24 us).
+// step takes 172 us against 352 before (Adam's 83 MB among them: 21 us).
 
 #include "pwa_internal.h"
 #include "tcgen05.cuh"
@@ -340,7 +340,7 @@ __device__ __forceinline__ long long w16Index(const MlpWeights& w, size_t i)
 // Adam on FP32 master weights; refreshes the BF16 copy.  Four parameters per
 // thread (the arrays come from the allocator, 16-byte aligned; every index into
 // the thread's own copies is known at compile time, so that they and the
-// weights' map stay in registers: 20 us for 3 M parameters, 24 with the map
+// weights' map stay in registers: 21 us for 3 M parameters, 24 with the map
 // indexed in local memory).  The moments'
 // fused multiply-adds are written out: a run's weights do not depend on which
 // product the compiler fuses.
