@@ -164,7 +164,7 @@ struct __align__(16) TriSlot {
 struct AccF32 {
 	typedef float2 Op;
 	typedef float Weight;
-	static constexpr int kUnroll = 2, kFold = 1 << 30;
+	static constexpr int kUnroll = 2, kFold = 0;
 	static constexpr bool kAsync = true;
 	float2 s[4][4];
 	__device__ void init()
@@ -283,7 +283,8 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 	const int bufOps = a.slices * stepOps * (kTwo ? 2 : 1);
 	Op* const buf0 = reinterpret_cast<Op*>(smemRaw);
 	const uint64_t chunk0 = (uint64_t)blockIdx.y * (unsigned)a.slices;
-	const bool mine = sl < a.slices && t < a.nTiles && chunk0 + sl < (uint64_t)a.chunks;
+	const bool inside = chunk0 + sl < (uint64_t)a.chunks;
+	const bool mine = sl < a.slices && t < a.nTiles && (Acc::kFold == 0 || inside);
 	Acc acc;
 	acc.init();
 
@@ -383,9 +384,11 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 #pragma unroll Acc::kUnroll
 			for (int q = 0; q < KT; ++q)
 				acc.template step<WT>(a0 + q * ld, b0 + q * ld, G, I - I0, J - I0, WT ? w0[q] : 0);
-			if (!more || (kb + KT) % Acc::kFold == 0) {
-				store(kb >= (uint32_t)Acc::kFold);
-				acc.init();
+			if constexpr (Acc::kFold > 0) {
+				if (!more || (kb + KT) % Acc::kFold == 0) {
+					store(kb >= (uint32_t)Acc::kFold);
+					acc.init();
+				}
 			}
 		}
 		if (!Acc::kAsync && more)
@@ -399,6 +402,8 @@ __global__ void __launch_bounds__(kTriThreads, 2) gramTriKernel(const In* __rest
 			wbuf[(round & 1) * a.slices * KT + tid] = (typename Acc::Weight)wNext;
 		cur ^= 1;
 	}
+	if (Acc::kFold == 0 && mine && inside)
+		store(false);
 }
 
 // Sums chunk partials (upper triangle) in FP64 and writes the full Hermitian
